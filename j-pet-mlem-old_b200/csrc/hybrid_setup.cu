@@ -199,34 +199,40 @@ __global__ void k_gather_frames(const Frame* __restrict__ frames, const int32_t*
 }
 }  // namespace
 
-cudaError_t order_frames_by_lor(const Frame* frames, int32_t n, int64_t n_lors, Frame* out,
-                                cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
+namespace {
+int lor_bits(int64_t n_lors) {
   int end_bit = 1;
   while (end_bit < 31 && ((int64_t)1 << end_bit) < n_lors) ++end_bit;
-  int32_t *keys = nullptr, *index = nullptr;
-  void* temp = nullptr;
+  return end_bit;
+}
+// keys, indices and their sorted copies, before CUB's own scratch
+size_t order_arrays_bytes(int32_t n) { return (4 * (size_t)n * sizeof(int32_t) + 255) & ~(size_t)255; }
+}  // namespace
+
+cudaError_t order_frames_scratch(int32_t n, int64_t n_lors, size_t* bytes, cudaStream_t st) {
+  int32_t* p = nullptr;
   size_t temp_bytes = 0;
-  cudaError_t e = cudaMalloc(&keys, 4 * (size_t)n * sizeof(int32_t));
-  if (e != cudaSuccess) return e;
-  index = keys + n;
+  const cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, p, p, p, p, n, 0,
+                                                        lor_bits(n_lors), st);
+  *bytes = order_arrays_bytes(n) + temp_bytes;
+  return e;
+}
+
+cudaError_t order_frames_by_lor(const Frame* frames, int32_t n, int64_t n_lors, Frame* out,
+                                char* scratch, size_t scratch_bytes, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  int32_t* keys = reinterpret_cast<int32_t*>(scratch);
+  int32_t* index = keys + n;
   int32_t* keys_out = keys + 2 * (size_t)n;
   int32_t* index_out = keys + 3 * (size_t)n;
+  size_t temp_bytes = scratch_bytes - order_arrays_bytes(n);
   k_lor_keys<<<grid_for(n), 256, 0, st>>>(frames, n, keys, index);
-  e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_out, index, index_out, n,
-                                      0, end_bit, st);
-  if (e == cudaSuccess) e = cudaMalloc(&temp, temp_bytes);
-  if (e == cudaSuccess)
-    e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, keys_out, index, index_out, n,
-                                        0, end_bit, st);
-  if (e == cudaSuccess) {
-    k_gather_frames<<<grid_for(n), 256, 0, st>>>(frames, index_out, n, out);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(temp);
-  cudaFree(keys);
-  return e;
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(scratch + order_arrays_bytes(n), temp_bytes, keys,
+                                                  keys_out, index, index_out, n, 0,
+                                                  lor_bits(n_lors), st);
+  if (e != cudaSuccess) return e;
+  k_gather_frames<<<grid_for(n), 256, 0, st>>>(frames, index_out, n, out);
+  return cudaGetLastError();
 }
 
 }  // namespace hybridmlem

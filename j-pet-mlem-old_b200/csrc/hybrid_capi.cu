@@ -61,6 +61,8 @@ struct hybrid_ctx {
   float* d_acc_t = nullptr;
   float* d_tmp = nullptr;  // boundary-layout staging
   float* d_spill = nullptr;  // per-warp weight slabs of k_mlem
+  int64_t n_lors_used = 0;  // LORs with pixel infos
+  WinSet win{};  // the windowed events of d_frames_iter (n_events 0: none)
   float* d_acc_user = nullptr;  // caller-owned accumulator (hybrid_set_accumulator)
   hybrid_stats stats{};
   std::string err;
@@ -97,20 +99,13 @@ template <typename T> void dfree(T*& p) {
 
 // Event-sized device buffers: from the context's pool, on its stream.
 template <typename T> cudaError_t ev_alloc(hybrid_ctx* ctx, T** p, size_t bytes) {
-  *p = nullptr;
   void* v = nullptr;
-  const cudaError_t e = ctx->pool ? cudaMallocFromPoolAsync(&v, bytes, ctx->pool, ctx->stream)
-                                  : cudaMalloc(&v, bytes);
-  if (e == cudaSuccess) *p = static_cast<T*>(v);
+  const cudaError_t e = EventMemory{ctx->pool, ctx->stream}.alloc(&v, bytes);
+  *p = static_cast<T*>(v);
   return e;
 }
 template <typename T> void ev_free(hybrid_ctx* ctx, T*& p) {
-  if (p) {
-    if (ctx->pool)
-      cudaFreeAsync(p, ctx->stream);
-    else
-      cudaFree(p);
-  }
+  EventMemory{ctx->pool, ctx->stream}.free(p);
   p = nullptr;
 }
 
@@ -172,46 +167,81 @@ void free_events(hybrid_ctx* ctx) {
   ev_free(ctx, ctx->d_frames);
   ev_free(ctx, ctx->d_frames_iter);
   ev_free(ctx, ctx->d_index);
+  ev_free(ctx, ctx->win.block);
+  ctx->win = WinSet{};
   ctx->n_events = 0;
   ctx->n_responses = 0;
 }
 
-// The iteration kernel takes the frame events in LOR order: the warps
-// resident at one time then work on a few LORs, whose pixel infos, weights
-// and image lines they share in L1 and L2 (205.4 against 207.8 ms per
-// iteration in response order on the big-barrel workload of 1e7 responses;
-// the order of the additions into the volume changes only the binary32
-// rounding of the sums).
-#ifndef HYBRID_LOR_ORDER
-#define HYBRID_LOR_ORDER 1
+// When the windowed iteration (k_win_project, k_win_back) takes the events.
+// It stages `entries` window entries, about 50 instructions each in both
+// kernels, besides 20 a voxel, where k_mlem spends 144 a voxel and nothing on
+// entries.  Measured on the big barrel (grid, responses: entries / voxels, ms
+// per iteration of k_mlem -> windowed): 60, 2e5: 0.74, 0.281 -> 0.286;
+// 100, 2e5: 0.73, 0.733 -> 0.645; 160, 2e5: 0.78, 2.22 -> 1.95; 80, 1e5: 1.4,
+// 0.246 -> 0.353; 100, 5e4: 1.7, 0.197 -> 0.357; 100, 2e6: 0.12, 6.97 -> 2.45;
+// so below HYBRID_WIN_RATIO entries a voxel.  Lists of fewer than
+// HYBRID_WIN_EVENTS_PER_LOR events per LOR with pixel infos lie beyond that
+// (5e4 to 1e5 responses there) and are not binned at all.
+#ifndef HYBRID_WIN_EVENTS_PER_LOR
+#define HYBRID_WIN_EVENTS_PER_LOR 8
 #endif
-int order_for_iterations(hybrid_ctx* ctx) {
+#ifndef HYBRID_WIN_RATIO
+#define HYBRID_WIN_RATIO 0.74
+#endif
+// Orders the frame events for the iterations: LOR by LOR, and within a LOR by
+// plane slab when the windows pay.  The order of the additions into the
+// volume changes only the binary32 rounding of the sums.
+int order_for_iterations(hybrid_ctx* ctx, int max_planes) {
   ev_free(ctx, ctx->d_frames_iter);
-  if (!HYBRID_LOR_ORDER || ctx->n_events <= 0) return STRIP_OK;
+  ev_free(ctx, ctx->win.block);
+  ctx->win = WinSet{};
+  if (ctx->n_events <= 0) return STRIP_OK;
   if (ctx->n_events > INT32_MAX)
     return fail(ctx, STRIP_E_INVALID, "more than 2^31 - 1 frame events");
   cudaError_t e = ev_alloc(ctx, &ctx->d_frames_iter, ctx->n_events * sizeof(Frame));
-  char* scratch = nullptr;
-  size_t bytes = 0;
   if (e == cudaSuccess)
-    e = order_frames_scratch((int32_t)ctx->n_events, ctx->n_lors, &bytes, ctx->stream);
-  if (e == cudaSuccess) e = ev_alloc(ctx, &scratch, bytes);
-  if (e == cudaSuccess)
-    e = order_frames_by_lor(ctx->d_frames, (int32_t)ctx->n_events, ctx->n_lors,
-                            ctx->d_frames_iter, scratch, bytes, ctx->stream);
-  ev_free(ctx, scratch);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    e = order_frames(ctx->g, geo_view(ctx), ctx->d_frames, (int32_t)ctx->n_events,
+                     ctx->n_events >= HYBRID_WIN_EVENTS_PER_LOR * ctx->n_lors_used
+                         ? plan_windows(ctx->g, max_planes) : WinPlan{},
+                     ctx->d_frames_iter, &ctx->win,
+                     EventMemory{ctx->pool, ctx->stream});
+  if (e == cudaSuccess &&
+      (double)ctx->win.entries >= HYBRID_WIN_RATIO * (double)ctx->stats.used_voxels) {
+    ev_free(ctx, ctx->win.block);
+    ctx->win = WinSet{};
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
-    ev_free(ctx, ctx->d_frames_iter);
+    free_events(ctx);
     return fail(ctx, e == cudaErrorMemoryAllocation ? STRIP_E_NOMEM : STRIP_E_CUDA,
-                "ordering the frame events by LOR: %s", cudaGetErrorString(e));
+                "ordering the frame events: %s", cudaGetErrorString(e));
   }
   return STRIP_OK;
 }
 
-const Frame* iter_frames(const hybrid_ctx* ctx) {
-  return ctx->d_frames_iter ? ctx->d_frames_iter : ctx->d_frames;
+// One backprojection of all events into acc (zeroed here), on the stream:
+// the windowed events, then the others and those the windows left over.
+int enqueue_mlem(hybrid_ctx* ctx, float* acc) {
+  const int blocks = ctx->sm_count * mlem_blocks_per_sm();
+  if (!ctx->d_spill) CK(cudaMalloc(&ctx->d_spill, mlem_spill_floats(blocks) * sizeof(float)));
+  CK(cudaMemsetAsync(acc, 0, ctx->n_voxels * sizeof(float), ctx->stream));
+  const WinSet& ws = ctx->win;
+  if (ws.n_events > 0) CK(cudaMemsetAsync(ws.counters, 0, 3 * sizeof(int32_t), ctx->stream));
+  CK(cudaEventRecord(ctx->ev0, ctx->stream));
+  if (ws.n_events > 0) {
+    launch_mlem_win(ctx->g, geo_view(ctx), ctx->d_sens, ws, ctx->d_rho_t, acc, ctx->sm_count,
+                    ctx->stream);
+    CK(cudaGetLastError());
+  }
+  if (ctx->n_events > 0)
+    launch_mlem(ctx->g, geo_view(ctx), ctx->d_sens, ctx->d_frames_iter + ws.n_events,
+                ctx->n_events - ws.n_events, ctx->d_frames_iter, ws.list,
+                ws.n_events > 0 ? ws.counters + 2 : nullptr, ctx->d_rho_t, acc, ctx->d_spill,
+                blocks, ctx->stream);
+  CK(cudaGetLastError());
+  CK(cudaEventRecord(ctx->ev1, ctx->stream));
+  return STRIP_OK;
 }
 
 void free_geometry(hybrid_ctx* ctx) {
@@ -239,10 +269,12 @@ int upload_geometry(hybrid_ctx* ctx, int32_t n_detectors, std::vector<float>& se
   free_geometry(ctx);
   std::vector<float4> md(n_lors);
   std::vector<float> len(n_lors);
+  int64_t used = 0;
   for (int64_t li = 0; li < n_lors; ++li) {
     const float* sg = seg.data() + li * 9;
     md[li] = make_float4(sg[4], sg[5], sg[6], sg[7]);
     len[li] = sg[8];
+    used += lend[li] > lbeg[li];
   }
   CK(cudaMalloc(&ctx->d_md, n_lors * sizeof(float4)));
   CK(cudaMalloc(&ctx->d_len, n_lors * sizeof(float)));
@@ -265,6 +297,7 @@ int upload_geometry(hybrid_ctx* ctx, int32_t n_detectors, std::vector<float>& se
   ctx->n_detectors = n_detectors;
   ctx->n_lors = n_lors;
   ctx->n_infos = n_infos;
+  ctx->n_lors_used = used;
   ctx->stats = hybrid_stats{};
   ctx->stats.n_lors = n_lors;
   ctx->stats.n_pixel_infos = n_infos;
@@ -324,7 +357,7 @@ int hybrid_ctx_create(const hybrid_setup* setup, int32_t device, hybrid_ctx** ou
         cudaMalloc(&ctx->d_tmp, vb) != cudaSuccess ||
         cudaMalloc(&ctx->d_sens, ctx->g.n_pixels * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&ctx->d_sens_acc, ctx->g.n_pixels * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&ctx->d_counts, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaMalloc(&ctx->d_counts, 4 * sizeof(unsigned long long)) != cudaSuccess) {
       rc = STRIP_E_NOMEM;
       break;
     }
@@ -626,6 +659,7 @@ int hybrid_set_responses(hybrid_ctx* ctx, const int16_t* first, const int16_t* s
   CKR(cudaMemcpyAsync(&last_keep, d_keep + (n - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   CKR(cudaStreamSynchronize(ctx->stream));
   const int64_t kept = last_off + last_keep;
+  unsigned long long counts[4] = {0, 0, 0, 0};
   if (kept > 0) {
     CKR(ev_alloc(ctx, &ctx->d_frames, kept * sizeof(Frame)));
     CKR(ev_alloc(ctx, &ctx->d_index, kept * sizeof(int64_t)));
@@ -633,7 +667,6 @@ int hybrid_set_responses(hybrid_ctx* ctx, const int16_t* first, const int16_t* s
     CKR(cudaGetLastError());
     launch_event_counts(ctx->d_frames, kept, ctx->d_counts, ctx->stream);
     CKR(cudaGetLastError());
-    unsigned long long counts[2] = {0, 0};
     CKR(cudaMemcpyAsync(counts, ctx->d_counts, sizeof counts, cudaMemcpyDeviceToHost, ctx->stream));
     CKR(cudaStreamSynchronize(ctx->stream));
     ctx->stats.used_pixels = (int64_t)counts[0];
@@ -643,7 +676,7 @@ int hybrid_set_responses(hybrid_ctx* ctx, const int16_t* first, const int16_t* s
   cleanup();
   ctx->n_events = kept;
   ctx->stats.n_events = kept;
-  return order_for_iterations(ctx);
+  return order_for_iterations(ctx, (int)counts[3]);
 }
 
 int hybrid_set_frames(hybrid_ctx* ctx, int64_t n, const int32_t* lor, const int64_t* info_begin,
@@ -688,14 +721,14 @@ int hybrid_set_frames(hybrid_ctx* ctx, int64_t n, const int32_t* lor, const int6
                      ctx->stream));
   launch_event_counts(ctx->d_frames, n, ctx->d_counts, ctx->stream);
   CK(cudaGetLastError());
-  unsigned long long counts[2] = {0, 0};
+  unsigned long long counts[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(counts, ctx->d_counts, sizeof counts, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->stats.used_pixels = (int64_t)counts[0];
   ctx->stats.used_voxels = (int64_t)counts[1];
   ctx->n_events = n;
   ctx->stats.n_events = n;
-  return order_for_iterations(ctx);
+  return order_for_iterations(ctx, (int)counts[3]);
 }
 
 int hybrid_get_frames(hybrid_ctx* ctx, int32_t* lor_index_out, int64_t* info_begin,
@@ -726,18 +759,9 @@ int hybrid_iterate(hybrid_ctx* ctx, int32_t n_iterations, hybrid_progress_cb pro
   if (n_iterations < 0) return fail(ctx, STRIP_E_INVALID, "negative iteration count");
   if (!ctx->have_sens) return fail(ctx, STRIP_E_STATE, "set the geometry and sensitivity first");
   CK(cudaSetDevice(ctx->device));
-  const size_t vb = ctx->n_voxels * sizeof(float);
-  const int blocks = ctx->sm_count * mlem_blocks_per_sm();
-  if (!ctx->d_spill) CK(cudaMalloc(&ctx->d_spill, mlem_spill_floats(blocks) * sizeof(float)));
   for (int32_t it = 0; it < n_iterations; ++it) {
     if (progress) progress(ctx->stats.iterations, 0, user);
-    CK(cudaMemsetAsync(ctx->d_acc_t, 0, vb, ctx->stream));
-    CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (ctx->n_events > 0)
-      launch_mlem(ctx->g, geo_view(ctx), ctx->d_sens, iter_frames(ctx), ctx->n_events, ctx->d_rho_t,
-                  ctx->d_acc_t, ctx->d_spill, blocks, ctx->stream);
-    CK(cudaGetLastError());
-    CK(cudaEventRecord(ctx->ev1, ctx->stream));
+    if (int rc = enqueue_mlem(ctx, ctx->d_acc_t)) return rc;
     CK(cudaEventSynchronize(ctx->ev1));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
@@ -760,15 +784,7 @@ int hybrid_accumulate(hybrid_ctx* ctx) {
   if (!ctx->have_sens) return fail(ctx, STRIP_E_STATE, "set the geometry and sensitivity first");
   CK(cudaSetDevice(ctx->device));
   float* acc = ctx->d_acc_user ? ctx->d_acc_user : ctx->d_acc_t;
-  const int blocks = ctx->sm_count * mlem_blocks_per_sm();
-  if (!ctx->d_spill) CK(cudaMalloc(&ctx->d_spill, mlem_spill_floats(blocks) * sizeof(float)));
-  CK(cudaMemsetAsync(acc, 0, ctx->n_voxels * sizeof(float), ctx->stream));
-  CK(cudaEventRecord(ctx->ev0, ctx->stream));
-  if (ctx->n_events > 0)
-    launch_mlem(ctx->g, geo_view(ctx), ctx->d_sens, iter_frames(ctx), ctx->n_events, ctx->d_rho_t,
-                acc, ctx->d_spill, blocks, ctx->stream);
-  CK(cudaGetLastError());
-  CK(cudaEventRecord(ctx->ev1, ctx->stream));
+  if (int rc = enqueue_mlem(ctx, acc)) return rc;
   CK(cudaEventSynchronize(ctx->ev1));
   float ms = 0;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

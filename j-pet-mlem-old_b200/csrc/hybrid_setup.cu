@@ -6,6 +6,8 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
+
 #include "hybrid_internal.h"
 
 namespace hybridmlem {
@@ -185,54 +187,241 @@ void launch_compact(const Frame* frames, const int32_t* keep, const int64_t* off
 }
 
 namespace {
-__global__ void k_lor_keys(const Frame* __restrict__ frames, int32_t n, int32_t* keys,
-                           int32_t* index) {
+
+// Sort keys: (LOR, plane slab); the largest key for an event no window takes
+// (counted).
+__global__ void k_order_keys(const Frame* __restrict__ frames, int32_t n, int64_t n_lors,
+                             const WinPlan w, uint64_t* keys, int32_t* index,
+                             int32_t* n_general) {
   for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    keys[i] = frames[i].lor;
+    const Frame f = frames[i];
+    uint64_t key = (uint64_t)f.lor;
+    if (w.planes > 0) {
+      const int rows = f.info_end - f.info_begin, planes = f.plane_end - f.plane_begin;
+      if (rows > 0 && planes > 0 && rows < (1 << kWinRowBits) && planes <= w.max_planes) {
+        key = key * w.n_slabs + f.plane_begin / w.tile_planes;
+      } else {
+        key = (uint64_t)n_lors * w.n_slabs;
+        atomicAdd(n_general, 1);
+      }
+    }
+    keys[i] = key;
     index[i] = i;
   }
 }
+
 __global__ void k_gather_frames(const Frame* __restrict__ frames, const int32_t* index,
                                 int32_t n, Frame* out) {
   for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     out[i] = frames[index[i]];
 }
+
+// flag[i] = 1 where a work item begins: at a new key and every
+// kWinItemEvents events of it.
+__global__ void k_item_flags(const uint64_t* __restrict__ keys, int32_t n, int32_t* flag) {
+  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint64_t k = keys[i];
+    int32_t lo = 0, m = i;  // first event of the key, in [0, i]
+    while (m > 0) {
+      const int32_t half = m >> 1;
+      if (keys[lo + half] < k) {
+        lo += half + 1;
+        m -= half + 1;
+      } else {
+        m = half;
+      }
+    }
+    flag[i] = (i - lo) % kWinItemEvents == 0 ? 1 : 0;
+  }
+}
+
+__global__ void k_item_begins(const int32_t* __restrict__ flag, const int64_t* __restrict__ offs,
+                              int32_t n, int32_t n_items, int32_t* begin) {
+  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    if (flag[i]) begin[offs[i]] = i;
+  if (blockIdx.x == 0 && threadIdx.x == 0) begin[n_items] = n;
+}
+
+// The items' pixel-info spans and numbers of tasks.  One warp per item.
+__global__ void k_item_boxes(const Frame* __restrict__ frames, const int32_t* __restrict__ begin,
+                             int32_t n_items, WinItem* items, int32_t* n_tasks) {
+  const int lane = threadIdx.x & 31;
+  const int32_t n_warps = gridDim.x * (blockDim.x >> 5);
+  for (int32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < n_items;
+       it += n_warps) {
+    const int32_t e0 = begin[it], e1 = begin[it + 1];
+    int i0 = 0x7FFFFFFF, i1 = 0;
+    for (int32_t e = e0 + lane; e < e1; e += 32) {
+      i0 = min(i0, frames[e].info_begin);
+      i1 = max(i1, frames[e].info_end);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      i0 = min(i0, __shfl_xor_sync(0xffffffffu, i0, o));
+      i1 = max(i1, __shfl_xor_sync(0xffffffffu, i1, o));
+    }
+    if (lane == 0) {
+      items[it] = WinItem{e0, e1, frames[e0].lor, i0, i1};
+      n_tasks[it] = (i1 - i0 + 63) / 64;
+    }
+  }
+}
+
+// The items' tasks, and the window entries they stage (planes by 32 and infos
+// by 2, as the kernels take them).  One warp per item.
+__global__ void k_item_tasks(const Frame* __restrict__ frames, const WinItem* __restrict__ items,
+                             const int64_t* __restrict__ offs, int32_t n_items, WinTask* tasks,
+                             unsigned long long* entries) {
+  const int lane = threadIdx.x & 31;
+  const int32_t n_warps = gridDim.x * (blockDim.x >> 5);
+  unsigned long long sum = 0;
+  for (int32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n_items;
+       i += n_warps) {
+    const WinItem it = items[i];
+    WinTask* out = tasks + offs[i];
+    for (int row0 = it.i0; row0 < it.i1; row0 += 64, ++out) {
+      int p0 = 0x7FFF, p1 = 0;
+      for (int32_t e = it.e0 + lane; e < it.e1; e += 32) {
+        const Frame f = frames[e];
+        if (f.info_begin < row0 + 64 && f.info_end > row0) {
+          p0 = min(p0, (int)f.plane_begin);
+          p1 = max(p1, (int)f.plane_end);
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        p0 = min(p0, __shfl_xor_sync(0xffffffffu, p0, o));
+        p1 = max(p1, __shfl_xor_sync(0xffffffffu, p1, o));
+      }
+      if (p1 <= p0) p0 = p1 = 0;
+      if (lane == 0) *out = WinTask{i, row0, (int16_t)p0, (int16_t)p1};
+      sum += (unsigned long long)((min(64, it.i1 - row0) + 1) & ~1) * ((p1 - p0 + 31) & ~31);
+    }
+  }
+  if (lane == 0 && sum) atomicAdd(entries, sum);
+}
+
 }  // namespace
 
-namespace {
-int lor_bits(int64_t n_lors) {
-  int end_bit = 1;
-  while (end_bit < 31 && ((int64_t)1 << end_bit) < n_lors) ++end_bit;
-  return end_bit;
-}
-// keys, indices and their sorted copies, before CUB's own scratch
-size_t order_arrays_bytes(int32_t n) { return (4 * (size_t)n * sizeof(int32_t) + 255) & ~(size_t)255; }
-}  // namespace
-
-cudaError_t order_frames_scratch(int32_t n, int64_t n_lors, size_t* bytes, cudaStream_t st) {
-  int32_t* p = nullptr;
-  size_t temp_bytes = 0;
-  const cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, p, p, p, p, n, 0,
-                                                        lor_bits(n_lors), st);
-  *bytes = order_arrays_bytes(n) + temp_bytes;
-  return e;
-}
-
-cudaError_t order_frames_by_lor(const Frame* frames, int32_t n, int64_t n_lors, Frame* out,
-                                char* scratch, size_t scratch_bytes, cudaStream_t st) {
+cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* frames, int32_t n,
+                         const WinPlan& plan, Frame* out, WinSet* ws, EventMemory mem) {
+  cudaStream_t st = mem.stream;
+  *ws = WinSet{};
+  ws->plan = plan;
   if (n <= 0) return cudaSuccess;
-  int32_t* keys = reinterpret_cast<int32_t*>(scratch);
-  int32_t* index = keys + n;
-  int32_t* keys_out = keys + 2 * (size_t)n;
-  int32_t* index_out = keys + 3 * (size_t)n;
-  size_t temp_bytes = scratch_bytes - order_arrays_bytes(n);
-  k_lor_keys<<<grid_for(n), 256, 0, st>>>(frames, n, keys, index);
-  cudaError_t e = cub::DeviceRadixSort::SortPairs(scratch + order_arrays_bytes(n), temp_bytes, keys,
-                                                  keys_out, index, index_out, n, 0,
-                                                  lor_bits(n_lors), st);
+  const bool win = plan.planes > 0;
+  const uint64_t n_keys = (uint64_t)geo.n_lors * (win ? (uint64_t)plan.n_slabs : 1) + 1;
+  int end_bit = 1;
+  while (end_bit < 64 && ((uint64_t)1 << end_bit) < n_keys) ++end_bit;
+  // one scratch block: keys and indices, sorted keys and indices, offsets,
+  // totals, CUB's own (sort and scan share it)
+  const size_t nn = ((size_t)n + 64) & ~(size_t)63;
+  size_t sort_bytes = 0, scan_bytes = 0;
+  uint64_t* kn = nullptr;
+  int32_t* in = nullptr;
+  int64_t* on = nullptr;
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, kn, kn, in, in, n, 0,
+                                                  end_bit, st);
+  if (e == cudaSuccess)
+    e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, in, on, n, st);
   if (e != cudaSuccess) return e;
+  const size_t temp_bytes = std::max(sort_bytes, scan_bytes);
+  void* block = nullptr;
+  e = mem.alloc(&block, nn * (8 + 8 + 8 + 4 + 4) + 256 + temp_bytes);
+  if (e != cudaSuccess) return e;
+  uint64_t* keys = static_cast<uint64_t*>(block);
+  uint64_t* keys_out = keys + nn;
+  int64_t* offs = reinterpret_cast<int64_t*>(keys_out + nn);
+  int32_t* index = reinterpret_cast<int32_t*>(offs + nn);
+  int32_t* index_out = index + nn;
+  unsigned long long* totals = reinterpret_cast<unsigned long long*>(index_out + nn);
+  int32_t* d_general = reinterpret_cast<int32_t*>(totals + 1);
+  void* temp = reinterpret_cast<char*>(totals) + 256;
+  void* items_tmp = nullptr;
+  auto done = [&](cudaError_t r) {
+    mem.free(items_tmp);
+    mem.free(block);
+    if (r != cudaSuccess) {
+      mem.free(ws->block);
+      *ws = WinSet{};
+    }
+    const cudaError_t s = cudaStreamSynchronize(st);
+    return r != cudaSuccess ? r : s;
+  };
+#define STEP(call)                              \
+  do {                                          \
+    e = (call);                                 \
+    if (e != cudaSuccess) return done(e);       \
+  } while (0)
+  // total of an exclusive scan: its last offset plus the last value
+  auto scan_total = [&](const int32_t* v, int32_t count, int64_t* total) {
+    size_t tb = temp_bytes;
+    cudaError_t r = cub::DeviceScan::ExclusiveSum(temp, tb, v, offs, count, st);
+    int64_t last = 0;
+    int32_t last_v = 0;
+    if (r == cudaSuccess)
+      r = cudaMemcpyAsync(&last, offs + (count - 1), 8, cudaMemcpyDeviceToHost, st);
+    if (r == cudaSuccess)
+      r = cudaMemcpyAsync(&last_v, v + (count - 1), 4, cudaMemcpyDeviceToHost, st);
+    if (r == cudaSuccess) r = cudaStreamSynchronize(st);
+    *total = last + last_v;
+    return r;
+  };
+  STEP(cudaMemsetAsync(totals, 0, 16, st));
+  k_order_keys<<<grid_for(n), 256, 0, st>>>(frames, n, geo.n_lors, plan, keys, index, d_general);
+  size_t tb = temp_bytes;
+  STEP(cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys_out, index, index_out, n, 0, end_bit,
+                                       st));
   k_gather_frames<<<grid_for(n), 256, 0, st>>>(frames, index_out, n, out);
-  return cudaGetLastError();
+  STEP(cudaGetLastError());
+  if (!win) return done(cudaSuccess);
+  int32_t n_general = 0;
+  STEP(cudaMemcpyAsync(&n_general, d_general, 4, cudaMemcpyDeviceToHost, st));
+  STEP(cudaStreamSynchronize(st));
+  const int32_t nf = n - n_general;
+  if (nf <= 0) return done(cudaSuccess);
+  int32_t* flag = index;  // the unsorted indices are done with
+  k_item_flags<<<grid_for(nf), 256, 0, st>>>(keys_out, nf, flag);
+  int64_t n_items = 0, n_tasks = 0;
+  STEP(scan_total(flag, nf, &n_items));
+  int32_t* begin = index_out;  // so are the sorted ones (n_items + 1 <= nn)
+  k_item_begins<<<grid_for(nf), 256, 0, st>>>(flag, offs, nf, (int32_t)n_items, begin);
+  STEP(mem.alloc(&items_tmp, (size_t)n_items * sizeof(WinItem)));
+  WinItem* items = static_cast<WinItem*>(items_tmp);
+  k_item_boxes<<<grid_for(n_items * 32), 256, 0, st>>>(out, begin, (int32_t)n_items, items, flag);
+  STEP(scan_total(flag, (int32_t)n_items, &n_tasks));
+  // task numbers are ints (with room for the warps' last looks): no windows
+  if (n_tasks > INT32_MAX - (1 << 20)) return done(cudaSuccess);
+  // the set's own block
+  auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t b_ev = up((size_t)nf * sizeof(WinEvent)), b_it = up((size_t)n_items * sizeof(WinItem)),
+               b_ta = up((size_t)n_tasks * sizeof(WinTask)), b_D = up((size_t)nf * sizeof(double)),
+               b_inv = up((size_t)nf * sizeof(float)), b_li = up((size_t)nf * sizeof(int32_t));
+  void* own_p = nullptr;
+  STEP(mem.alloc(&own_p, b_ev + b_it + b_ta + b_D + b_inv + b_li + 256));
+  char* own = static_cast<char*>(own_p);
+  ws->block = own;
+  STEP(cudaMemcpyAsync(own + b_ev, items, (size_t)n_items * sizeof(WinItem),
+                       cudaMemcpyDeviceToDevice, st));
+  ws->events = reinterpret_cast<WinEvent*>(own);
+  ws->items = reinterpret_cast<WinItem*>(own + b_ev);
+  ws->tasks = reinterpret_cast<WinTask*>(own + b_ev + b_it);
+  ws->D = reinterpret_cast<double*>(own + b_ev + b_it + b_ta);
+  ws->inv = reinterpret_cast<float*>(own + b_ev + b_it + b_ta + b_D);
+  ws->list = reinterpret_cast<int32_t*>(own + b_ev + b_it + b_ta + b_D + b_inv);
+  ws->counters = reinterpret_cast<int32_t*>(own + b_ev + b_it + b_ta + b_D + b_inv + b_li);
+  ws->n_events = nf;
+  ws->n_items = (int32_t)n_items;
+  ws->n_tasks = (int32_t)n_tasks;
+  STEP(cudaMemsetAsync(ws->D, 0, b_D, st));
+  k_item_tasks<<<grid_for(n_items * 32), 256, 0, st>>>(out, ws->items, offs, (int32_t)n_items,
+                                                      ws->tasks, totals);
+  launch_win_events(g, geo, out, nf, ws->events, st);
+  STEP(cudaGetLastError());
+  unsigned long long entries = 0;
+  STEP(cudaMemcpyAsync(&entries, totals, 8, cudaMemcpyDeviceToHost, st));
+  STEP(cudaStreamSynchronize(st));
+  ws->entries = (int64_t)entries;
+  return done(cudaSuccess);
+#undef STEP
 }
 
 }  // namespace hybridmlem

@@ -105,13 +105,42 @@ KernelF make_kernel(double sigma_z, double sigma_dl, float pw) {
   return k;
 }
 
+// The kernel constants per kc^2, so that rsqrt gives kc / sqrt(a'Sa); and with
+// d = log2 of the rounded q over the true one, pixel j of a run of l + 1
+// carries d j (j - 1) / 2: K0 takes 2^(d (l^2 / 8 - w)) and R0 2^(d (1 - l) / 2),
+// which leaves d ((j - l / 2)^2 / 2 - w), w = sigma_z^2 / 4 its mean over the
+// Gaussian (pixels).
+PairConst make_pair_const(const ScannerF& s, const KernelF& k) {
+  PairConst c;
+  c.nzero = -0.0f;
+  c.C = 2.0f * s.ipsz;
+  const double per_px2 = (double)s.inv2z * s.inv_pw * s.inv_pw;
+  c.c9 = (float)(9.0 * per_px2);
+  c.nk4 = (float)(-4.0 * s.ipsdl * per_px2);
+  const double kc2 = (double)k.kc * k.kc;
+  c.na4 = (float)(2.0 * k.ipsz / kc2);
+  c.na2 = (float)(4.0 * k.ipsdl / kc2);
+  c.nb4 = (float)(2.0 * k.ipsz * s.R * s.R / kc2);
+  c.cd = -2.0f * kLog2e * k.ipsdl;
+  c.c1 = k.c1;
+  c.r1 = k.r1;
+  c.q = k.q;
+  const double d = std::log2((double)k.q) - 2.0 * (double)k.c1 * s.pw * s.pw;
+  c.r0 = (float)((double)k.c1 * s.pw * s.pw + 0.5 * d);
+  c.dh = (float)(-0.5 * d);
+  c.d8 = (float)(0.125 * d);
+  c.d0 = (float)(-0.25 * d / ((double)k.ipsz * s.pw * s.pw));
+  return c;
+}
+
+bool pair_const_ok(const PairConst& c) {
+  auto in = [](float v, float lo, float hi) { return v > lo && v < hi; };
+  return in(c.na4, 1e-25f, 1e25f) && in(c.na2, 1e-25f, 1e25f) && in(c.nb4, 1e-25f, 1e25f) &&
+         in(c.q, 1e-6f, 2.0f) && in(c.c9, 1e-25f, 1e25f) && std::isfinite(c.d0);
+}
+
 }  // namespace stripmlem
 
-// Each work item's events ordered for the column-major windows' banks
-// (k_item_order; a build-time switch for comparisons).
-#ifndef STRIP_ITEM_ORDER
-#define STRIP_ITEM_ORDER 1
-#endif
 // With the item size chosen per binning, the last STRIP_TAIL_WAVES waves of
 // a subset's work items (by events, one wave = two CTAs per SM, each with a
 // full item) are cut into STRIP_TAIL_PIECES pieces each, so the launch's last
@@ -183,8 +212,13 @@ Tiling choose_tiling(const strip_ctx* ctx, int max_w, int max_h) {
     if (HX >= HY) HX = HX * 3 / 4; else HY = HY * 3 / 4;
   }
   // column-major windows where they fit the same budget (fewer shared-memory
-  // bank conflicts in the walks)
-  t.cs = tile_column_stride(t.WXmax, t.WYmax, budget);
+  // bank conflicts in the walks); the row-pair kernels, which run there, need
+  // the closed form to settle every row and the kernel's constants in range
+  const bool pairs =
+      ctx->s.min_closed_hw == 0.0f &&
+      pair_const_ok(make_pair_const(
+          ctx->s, make_kernel(ctx->g.sigma_z, ctx->g.sigma_dl, ctx->s.pw)));
+  t.cs = pairs ? tile_column_stride(t.WXmax, t.WYmax, budget) : 0;
   if (t.cs) t.smem_bytes = 2 * t.WXmax * t.cs * 4;
   t.ntx = (n_z + t.TX - 1) / t.TX;
   t.nty = (n_y + t.TY - 1) / t.TY;
@@ -207,7 +241,9 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   unsigned long long* d_hist = nullptr;
   float *ozu = nullptr, *ozd = nullptr, *odl = nullptr;
   int64_t* operm = nullptr;
+  EventPack* packs = nullptr;
   auto cleanup = [&]() {
+    ev_free(ctx, packs);
     ev_free(ctx, boxes);
     ev_free(ctx, keys);
     dfree(d_wh);
@@ -355,7 +391,7 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   }
   // column-major windows: each item's events in quads of middle-row classes
   // (k_item_order); the binned arrays are replaced by the ordered ones
-  if (t.cs != 0 && !items.empty() && STRIP_ITEM_ORDER) {
+  if (t.cs != 0 && !items.empty()) {
     // the boxes and keys are done with: the pool hands their memory to the
     // ordered arrays
     ev_free(ctx, boxes);
@@ -366,9 +402,10 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
     if (e == cudaSuccess) e = ev_alloc(ctx, &qzd, nb * sizeof(float));
     if (e == cudaSuccess) e = ev_alloc(ctx, &qdl, nb * sizeof(float));
     if (e == cudaSuccess) e = ev_alloc(ctx, &qperm, nb * sizeof(int64_t));
+    if (e == cudaSuccess) e = ev_alloc(ctx, &packs, nb * sizeof(EventPack));
     if (e == cudaSuccess)
       e = launch_item_order(ctx->s, t, d_items, (int)items.size(), ozu, ozd, odl, operm, qzu,
-                            qzd, qdl, qperm, st);
+                            qzd, qdl, qperm, packs, st);
     if (e != cudaSuccess) {
       ev_free(ctx, qzu);
       ev_free(ctx, qzd);
@@ -405,8 +442,11 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   ev_free(ctx, ctx->d_zd);
   ev_free(ctx, ctx->d_dl);
   ev_free(ctx, ctx->d_perm);
+  ev_free(ctx, ctx->d_packs);
   dfree(ctx->d_items);
   dfree(ctx->d_item_hist);
+  ctx->d_packs = packs;
+  packs = nullptr;
   ctx->d_item_hist = d_ihist;
   ctx->d_zu = ozu;
   ctx->d_zd = ozd;
@@ -475,6 +515,8 @@ LaunchArgs base_args(strip_ctx* ctx) {
   a.zd = ctx->d_zd;
   a.dl = ctx->d_dl;
   a.perm = ctx->d_perm;
+  a.packs = ctx->d_packs;
+  a.pc = make_pair_const(a.s, a.k);
   a.rho = ctx->d_rho;
   a.acc = ctx->d_acc;
   a.status = ctx->d_status;
@@ -624,6 +666,7 @@ int strip_ctx_destroy(strip_ctx* ctx) {
   ev_free(ctx, ctx->d_zd);
   ev_free(ctx, ctx->d_dl);
   ev_free(ctx, ctx->d_perm);
+  ev_free(ctx, ctx->d_packs);
   dfree(ctx->d_items);
   dfree(ctx->d_item_hist);
   dfree(ctx->d_fallback);
@@ -903,6 +946,7 @@ int forward_dev(strip_ctx* ctx, const float* d_rho, double sz, double sdl,
   CK(cudaMemsetAsync(d_y, 0, ctx->n_events * sizeof(double), ctx->stream));
   LaunchArgs a = base_args(ctx);
   a.k = make_kernel(sz, sdl, ctx->s.pw);
+  a.pc = make_pair_const(a.s, a.k);
   a.rho = d_rho;
   a.sens = (mode == STRIP_MODE_GPU) ? ctx->d_sens5 : nullptr;
   a.y_out = d_y;
@@ -921,6 +965,7 @@ int adjoint_dev(strip_ctx* ctx, const double* d_w, double sz, double sdl,
                            ctx->stream));
   LaunchArgs a = base_args(ctx);
   a.k = make_kernel(sz, sdl, ctx->s.pw);
+  a.pc = make_pair_const(a.s, a.k);
   a.acc = d_g;
   a.wf_in = ctx->d_wbin;
   // GaussianKernel values are at most kc / sqrt(2 R^2 ipsz): E <= 1 and
@@ -938,6 +983,7 @@ int grad_dev(strip_ctx* ctx, const float* d_rho, const double* d_w, double sz,
   CK(cudaMemsetAsync(d_out2, 0, 2 * sizeof(double), ctx->stream));
   LaunchArgs a = base_args(ctx);
   a.k = make_kernel(sz, sdl, ctx->s.pw);
+  a.pc = make_pair_const(a.s, a.k);
   a.rho = d_rho;
   a.w_in = d_w;
   a.grad_out = d_out2;

@@ -42,6 +42,7 @@ struct strip_ctx {
   float* d_zd = nullptr;
   float* d_dl = nullptr;
   int64_t* d_perm = nullptr;
+  stripmlem::EventPack* d_packs = nullptr;  // set-up events (column-major windows)
   int n_subsets = 0;
   stripmlem::Tiling t{};
   int max_w = 0, max_h = 0;

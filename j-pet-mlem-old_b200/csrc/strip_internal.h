@@ -95,6 +95,30 @@ enum Op {
 cudaError_t launch_split_triples(const float* aos, int64_t n, float* zu, float* zd,
                                  float* dl, cudaStream_t st);
 
+// A set-up event: tan, y, z, sec and the clamped box (columns and rows lie in
+// [0, 32767]) in two words.  The ellipse's A, B, C follow from tan and sec (and
+// the scanner) by the same rounded binary32 operations as in event_setup.
+struct EventPack {
+  float tan, y, z, sec;
+  unsigned x, yb;  // tlx | brx << 16, tly | bry << 16
+};
+
+// Launch constants of the row-pair kernels (strip_pairs.cu): the closed-form
+// ends of the pixel runs (the geometry's sigmas) and the kernel values (the
+// model's).
+struct PairConst {
+  float nzero;          // -0
+  float C;              // 2 / sigma_z^2, as event_setup
+  float c9, nk4;        // hw^2 = c9 + nk4 sec^2 dy^2, in pixels^2
+  float na4, na2, nb4;  // a'Sa / kc^2 = (na4 sec^4 + na2 sec^2 tan^2) yp^2 + nb4 sec^4
+  float cd, c1;         // log2 E = c1 t^2 + cd sec^2 dy^2
+  float r1, r0, q;      // ratio 2^(r1 t + r0), ratio of ratios
+  float d8, d0, dh;     // centring of q's rounding error (make_pair_const)
+};
+// Whether the row-pair kernels can take the kernel's constants.
+bool pair_const_ok(const PairConst& c);
+PairConst make_pair_const(const ScannerF& s, const KernelF& k);
+
 struct LaunchArgs {
   ScannerF s;
   KernelF k;          // kernel constants (model sigmas)
@@ -102,6 +126,8 @@ struct LaunchArgs {
   const float* zu;    // events, binned order
   const float* zd;
   const float* dl;
+  const EventPack* packs;  // the same, set up (column-major windows)
+  PairConst pc;
   const int64_t* perm;   // binned position -> caller's event index
   const float* rho;      // image
   const float* sens;     // pixel sensitivity (gpu mode) or null
@@ -178,11 +204,18 @@ cudaError_t launch_bin_scatter(const int* keys, int64_t n, const float* zu,
 cudaError_t launch_tile(int op, int mode, int accum, const LaunchArgs& a,
                         cudaStream_t st);
 // The events of each work item (binned arrays zu.. perm) reordered into
-// ozu.. operm for the column-major windows' banks (k_item_order).
+// ozu.. operm for the column-major windows' banks (k_item_order), and set up
+// into packs.
 cudaError_t launch_item_order(const ScannerF& s, const Tiling& t, const WorkItem* items,
                               int n_items, const float* zu, const float* zd, const float* dl,
                               const int64_t* perm, float* ozu, float* ozd, float* odl,
-                              int64_t* operm, cudaStream_t st);
+                              int64_t* operm, EventPack* packs, cudaStream_t st);
+// GaussianKernel over column-major windows (strip_pairs.cu).
+cudaError_t launch_pair_tile(int op, int accum, const LaunchArgs& a, cudaStream_t st);
+cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows);
+cudaError_t launch_pair_batch(int accum, const BatchArgs& b, const BatchItem* items, int n_items,
+                              int* counter, int smem_bytes, int max_rows, int sm_count,
+                              cudaStream_t st);
 cudaError_t launch_global(int op, int mode, int accum, const LaunchArgs& a,
                           cudaStream_t st);
 // rho_j <- rho_j * acc_j * scale, or acc_j * scale when the accumulator holds

@@ -2,7 +2,9 @@
 //
 //   k_event_boxes / k_bin_keys / k_bin_scatter   one-time binning of the events
 //       into image tiles (events are iteration-invariant, so this is paid once)
-//   k_tile      the hot kernel: one CTA per (tile, event chunk) work item.  The
+//   k_tile      the tile kernel (row-major windows, the AnalyticKernel and the
+//       sigma gradient; the GaussianKernel over column-major windows, the
+//       common case, is strip_pairs.cu's): one CTA per (tile, event chunk) work item.  The
 //       tile's window of the image (tile + halo) is staged in shared memory
 //       next to a shared-memory backprojection accumulator.  A warp takes one
 //       event at a time:
@@ -27,12 +29,12 @@
 
 #include "strip_internal.h"
 #include "strip_rows.cuh"
+#include "strip_tile.cuh"
 
 namespace stripmlem {
 
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 // Threads of a tile CTA whose windows leave room for two CTAs per SM.
@@ -40,15 +42,10 @@ constexpr int kWarps = kThreads / 32;
 #define STRIP_TILE_THREADS 512
 #endif
 constexpr int kTileThreads = STRIP_TILE_THREADS;
-// Tile kernels whose shared-memory windows leave room for one CTA per SM
-// run 1024-thread CTAs (32 warps, 64 registers each), so the SM keeps as
-// many resident warps as with two 512-thread CTAs.
-constexpr int kWideThreads = 1024;
 // Column-major tile windows where they fit (tile_column_stride).
 #ifndef STRIP_COLUMN_MAJOR
 #define STRIP_COLUMN_MAJOR 1
 #endif
-constexpr int kMaxWarps = kWideThreads / 32;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -56,19 +53,6 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// A set-up event as a warp holds it until its turn: tan, y, z, sec and the
-// clamped box (columns and rows lie in [0, 32767]) in two words.  The
-// ellipse's A, B, C follow from tan and sec (and the scanner) by the same
-// rounded binary32 operations as in event_setup, so they are formed again
-// when the event is taken (fewer registers held through the walks).
-struct EventPack {
-  float tan, y, z, sec;
-  unsigned x, yb;  // tlx | brx << 16, tly | bry << 16
-};
-__device__ __forceinline__ EventPack pack_event(const EventF& e) {
-  return EventPack{e.tan, e.y, e.z, e.sec, (unsigned)e.tlx | ((unsigned)e.brx << 16),
-                   (unsigned)e.tly | ((unsigned)e.bry << 16)};
-}
 __device__ __forceinline__ EventF shfl_event(const ScannerF& s, const EventPack& m, int src) {
   EventF e;
   e.tan = __shfl_sync(kFull, m.tan, src);
@@ -89,35 +73,6 @@ __device__ __forceinline__ EventF shfl_event(const ScannerF& s, const EventPack&
   return e;
 }
 
-// Accumulation of the per-row partial sums of D_e within a lane.
-template <int ACC>
-struct RowSum;
-template <>
-struct RowSum<STRIP_ACCUM_FP32> {
-  float s = 0.0f;
-  __device__ __forceinline__ void add(float x) { s += x; }
-  __device__ __forceinline__ double total() const { return (double)s; }
-};
-template <>
-struct RowSum<STRIP_ACCUM_KAHAN> {
-  float s = 0.0f, c = 0.0f;
-  __device__ __forceinline__ void add(float x) {
-    const float yv = __fsub_rn(x, c);
-    const float t = __fadd_rn(s, yv);
-    c = __fsub_rn(__fsub_rn(t, s), yv);
-    s = t;
-  }
-  __device__ __forceinline__ double total() const {
-    return (double)s - (double)c;
-  }
-};
-template <>
-struct RowSum<STRIP_ACCUM_FP64> {
-  double s = 0.0;
-  __device__ __forceinline__ void add(float x) { s += (double)x; }
-  __device__ __forceinline__ double total() const { return s; }
-};
-
 // Binary32 -> integer by a power-of-two addend: for 0 <= x * s < 2^23 the
 // bits of x * s + 2^23 (one FFMA, round to nearest) minus those of 2^23 are
 // round(x * s); for |x * s| < 2^22 the same with 1.5 * 2^23 gives the
@@ -128,18 +83,6 @@ constexpr float kMagicSigned = 12582912.0f;
 constexpr unsigned kMagicSignedBits = 0x4B400000u;
 __device__ __forceinline__ unsigned to_fixed(float x, float s) {
   return __float_as_uint(fmaf(x, s, kMagic)) - kMagicBits;
-}
-
-// Shared-memory access by 32-bit shared-space byte address: the walks below
-// advance one address register per step and let the loads and atomics use
-// immediate offsets.
-__device__ __forceinline__ float lds32(uint32_t addr) {
-  float v;
-  asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void red_shared_add(uint32_t addr, unsigned v) {
-  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
 // Row of rank i among an event's H box rows, ranked middle-out: the centre
@@ -159,15 +102,6 @@ __device__ __forceinline__ int ranked_row(int H, int i) {
 // The fixed-point kinds use native 32-bit integer shared atomics; the scale
 // `fixed_unit` is a power of two chosen per work item so that no sum wraps.
 enum AccKind { kAccF32 = 0, kAccU32 = 1, kAccU32Cvt = 2, kAccS32 = 3, kAccU32Unw = 4 };
-
-// Per-CTA state of the work item in flight: the unweighted window's
-// fixed-point budget (units of 2^8), the item's sum of 1 / D_e, and the
-// events the unweighted window had no room for (bit i: event begin + i).
-constexpr unsigned kBudgetUnits = (unsigned)(kFixedBudget / 256.0f);
-__shared__ unsigned s_fx_budget;
-__shared__ float s_item_rsum;
-__shared__ unsigned s_fb_bits[kMaxItemEvents / 32];
-__shared__ int s_fb_n;
 
 // A tile's window in shared memory: row-major with row stride WS (CS = 0), or
 // column-major with column stride CS words (a multiple of 32).  Column-major,
@@ -827,36 +761,6 @@ __device__ __forceinline__ RowTables warp_tables(char* base, int cap, int warp) 
   return row_tables_at(base + (size_t)warp * row_table_bytes(cap), cap);
 }
 
-// Fixed-point scale of an adjoint work item: every addend is K_j w_e with
-// K_j <= a.kbound (the GaussianKernel's bound, E <= 1 and a'Sa >= 2 R^2 ipsz)
-// and |w_e| <= W, the item's largest weight, so with B = kbound * W the
-// scale 2^s keeps each addend below 2^22 and the item's sum below 2^31.
-__device__ int adjoint_shift(const LaunchArgs& a, const WorkItem& it, int lane) {
-  __shared__ float s_wmax[kMaxWarps];
-  __shared__ int s_shift;
-  float m = 0.0f;
-  for (int64_t i = it.begin + threadIdx.x; i < it.begin + it.count;
-       i += blockDim.x)
-    m = fmaxf(m, fabsf(a.wf_in[i]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(kFull, m, o));
-  if (lane == 0) s_wmax[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float W = 0.0f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) W = fmaxf(W, s_wmax[i]);
-    const float B = a.kbound * W * 1.0001f;
-    const float n = (float)it.count + (float)(it.count >> 7) + 1.0f;
-    const float lim = fminf(4194304.0f, 2147483648.0f / n);
-    int sh = 0;
-    if (B > 0.0f && B < 3.0e38f)
-      sh = (int)floorf(log2f(lim / B)) - 1;
-    s_shift = max(-120, min(120, sh));
-  }
-  __syncthreads();
-  return s_shift;
-}
-
 // The events of a work item: warps pull groups of a.grab (1..32) events from
 // a shared counter until the item is done (lanes < a.grab set the group's
 // events up in parallel).  With `only`, just the events whose bit is set:
@@ -910,23 +814,6 @@ __device__ __forceinline__ void run_item(const LaunchArgs& a, const WorkItem& it
   }
   if (OP == OP_MLEM && (lane & (LPE - 1)) == 0 && !only && rsum != 0.0f)
     atomicAdd(&s_item_rsum, rsum);
-}
-
-// Sum of v over the CTA, returned to every thread (two barriers).
-__device__ __forceinline__ float block_sum(float v) {
-  __shared__ float s_part[kMaxWarps];
-  __shared__ float s_total;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_part[w];
-    s_total = t;
-  }
-  __syncthreads();
-  return s_total;
 }
 
 // One work item on the whole CTA: stage the window, run the events, flush.
@@ -1326,41 +1213,53 @@ __global__ void k_bin_scatter(const int* keys, int64_t n, const float* zu,
 // middle rows are v, v + 16, v + 8 and v + 24 mod 32 (the half-warp pairs of
 // MLEM take (v, v + 16) and (v + 8, v + 24), the quarter-warps of the
 // forward and adjoint all four), then pairs (v, v + 16) of the events left,
-// then the rest.  One CTA per item; the order within a middle-row class is
-// that of the atomics.  The results change only by the order of the binary32
+// then the rest.  Within a middle-row class the events go by size (box rows,
+// eight steps of a sixteenth of the tallest), so that the events of a quad are
+// alike and their walks equally long.  One CTA per item; the order within a
+// class and size is that of the atomics.  The results change only by the order of the binary32
 // sums.
 __global__ void k_item_order(ScannerF s, Tiling t, const WorkItem* __restrict__ items,
                              const float* __restrict__ zu, const float* __restrict__ zd,
                              const float* __restrict__ dl, const int64_t* __restrict__ perm,
-                             float* ozu, float* ozd, float* odl, int64_t* operm) {
-  __shared__ int s_n[32], s_cnt[32];
+                             float* ozu, float* ozd, float* odl, int64_t* operm,
+                             EventPack* packs) {
+  // 32 middle-row classes x 8 sizes: counts, then first ranks within the class
+  __shared__ int s_n[32][8], s_first[32][8], s_all[32];
   __shared__ int s_q[32], s_qbase[32], s_p[32], s_pbase[32], s_sbase[32];
   const WorkItem it = items[blockIdx.x];
   int wx0, wy0, wx1, wy1;
   tile_window(t, s.n_z, s.n_y, it.tile, wx0, wy0, wx1, wy1);
-  if (threadIdx.x < 32) {
-    s_n[threadIdx.x] = 0;
-    s_cnt[threadIdx.x] = 0;
-  }
+  for (int k = threadIdx.x; k < 256; k += blockDim.x) s_n[k >> 3][k & 7] = 0;
   __syncthreads();
-  auto cls = [&](int64_t i) {
-    EventF e;
+  auto cls = [&](int64_t i, EventF& e) {
     event_setup(s, zu[i], zd[i], dl[i], e);
-    return (e.tly + ((e.bry - e.tly - 1) >> 1) - wy0) & 31;
+    const int H = e.bry - e.tly;
+    const int size = min(7, (t.max_rows - H) * 16 / t.max_rows);
+    return ((e.tly + (H >> 1) - wy0) & 31) * 8 + size;
   };
   // class counts and, below, ranks: one shared atomic per class and warp
   // (lanes of a class found by __match_any_sync)
   const int lane = threadIdx.x & 31;
   const int n_round = (it.count + blockDim.x - 1) / blockDim.x * blockDim.x;
   for (int k = threadIdx.x; k < n_round; k += blockDim.x) {
-    const int v = k < it.count ? cls(it.begin + k) : -1;
+    EventF e;
+    const int v = k < it.count ? cls(it.begin + k, e) : -1;
     const unsigned peers = __match_any_sync(kFull, v);
-    if (v >= 0 && lane == __ffs(peers) - 1) atomicAdd(&s_n[v], __popc(peers));
+    if (v >= 0 && lane == __ffs(peers) - 1) atomicAdd(&s_n[0][0] + v, __popc(peers));
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    int first = 0;
+    for (int z = 0; z < 8; ++z) {
+      s_first[threadIdx.x][z] = first;
+      first += s_n[threadIdx.x][z];
+    }
+    s_all[threadIdx.x] = first;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     int left[32];
-    for (int v = 0; v < 32; ++v) left[v] = s_n[v];
+    for (int v = 0; v < 32; ++v) left[v] = s_all[v];
     int pos = 0;
     for (int v = 0; v < 8; ++v) {  // quads: v, v + 16, v + 8, v + 24
       const int c[4] = {v, v + 16, v + 8, v + 24};
@@ -1389,13 +1288,15 @@ __global__ void k_item_order(ScannerF s, Tiling t, const WorkItem* __restrict__ 
   __syncthreads();
   for (int k = threadIdx.x; k < n_round; k += blockDim.x) {
     const int64_t i = it.begin + k;
-    const int v = k < it.count ? cls(i) : -1;
-    const unsigned peers = __match_any_sync(kFull, v);
+    EventF e;
+    const int vz = k < it.count ? cls(i, e) : -1;
+    const unsigned peers = __match_any_sync(kFull, vz);
     const int leader = __ffs(peers) - 1;
     int r0 = 0;
-    if (v >= 0 && lane == leader) r0 = atomicAdd(&s_cnt[v], __popc(peers));
+    if (vz >= 0 && lane == leader) r0 = atomicAdd(&s_first[0][0] + vz, __popc(peers));
     r0 = __shfl_sync(kFull, r0, leader);
-    if (v < 0) continue;
+    if (vz < 0) continue;
+    const int v = vz >> 3;
     const int r = r0 + __popc(peers & ((1u << lane) - 1u));
     const int q = s_q[v], p = s_p[v];
     const int at = r < q ? s_qbase[v] + 4 * r
@@ -1405,6 +1306,7 @@ __global__ void k_item_order(ScannerF s, Tiling t, const WorkItem* __restrict__ 
     ozd[o] = zd[i];
     odl[o] = dl[i];
     operm[o] = perm[i];
+    packs[o] = pack_event(e);
   }
 }
 
@@ -1559,20 +1461,30 @@ int grid_for(int64_t n, int per_block = kThreads, int cap = 148 * 16) {
 
 constexpr int kSetsCap = 64;
 
-template <int OP, int MODE, int ACC, int LPE>
-cudaError_t launch_tile_lpe(const LaunchArgs& a, cudaStream_t st) {
+// Column-major windows reach this file's kernels for the AnalyticKernel and
+// the sigma gradient only (the others: launch_pair_tile).
+template <int OP, int MODE>
+constexpr bool column_major() { return MODE != STRIP_MODE_CPU || OP == OP_GRAD; }
+
+template <int OP, int MODE, int ACC, int LPE, int CS>
+cudaError_t launch_tile_cs(const LaunchArgs& a, cudaStream_t st) {
   const int smem = a.t.smem_bytes / 2 * tile_windows<OP>();
   const bool wide = smem > kNarrowSmemBytes;  // one CTA per SM: 1024 threads
-  auto fn = a.t.cs == kColumnStride
-                ? (wide ? k_tile<OP, MODE, ACC, kWideThreads, LPE, kColumnStride>
-                        : k_tile<OP, MODE, ACC, kTileThreads, LPE, kColumnStride>)
-                : (wide ? k_tile<OP, MODE, ACC, kWideThreads, LPE, 0>
-                        : k_tile<OP, MODE, ACC, kTileThreads, LPE, 0>);
+  auto fn = wide ? k_tile<OP, MODE, ACC, kWideThreads, LPE, CS>
+                 : k_tile<OP, MODE, ACC, kTileThreads, LPE, CS>;
   cudaError_t err = cudaFuncSetAttribute(
       fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;
   fn<<<a.n_items, wide ? kWideThreads : kTileThreads, smem, st>>>(a);
   return cudaGetLastError();
+}
+
+template <int OP, int MODE, int ACC, int LPE>
+cudaError_t launch_tile_lpe(const LaunchArgs& a, cudaStream_t st) {
+  if constexpr (column_major<OP, MODE>()) {
+    if (a.t.cs == kColumnStride) return launch_tile_cs<OP, MODE, ACC, LPE, kColumnStride>(a, st);
+  }
+  return launch_tile_cs<OP, MODE, ACC, LPE, 0>(a, st);
 }
 
 template <int OP, int MODE, int ACC>
@@ -1623,6 +1535,8 @@ int tile_column_stride(int WXmax, int WYmax, int budget) {
 cudaError_t launch_tile(int op, int mode, int accum, const LaunchArgs& a,
                         cudaStream_t st) {
   if (a.n_items <= 0) return cudaSuccess;
+  if (mode == STRIP_MODE_CPU && a.t.cs == kColumnStride && op != OP_GRAD)
+    return launch_pair_tile(op, accum, a, st);
   switch (op) {
     case OP_MLEM:
       STRIP_DISPATCH(launch_tile_t, OP_MLEM, mode, accum, a, st);
@@ -1658,6 +1572,7 @@ cudaError_t launch_global(int op, int mode, int accum, const LaunchArgs& a,
 
 template <int THREADS, int CS, class F>
 cudaError_t with_tile_batch_t(int mode, int accum, bool half, F&& pick) {
+  if constexpr (CS == 0)
   if (mode == STRIP_MODE_CPU) {
     constexpr int H = lanes_per_event<OP_MLEM, STRIP_MODE_CPU>();
     if (half) {
@@ -1697,6 +1612,8 @@ cudaError_t with_tile_batch(int mode, int accum, int smem_bytes, int max_rows, i
 }
 
 cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max_rows, int cs) {
+  if (mode == STRIP_MODE_CPU && cs == kColumnStride)
+    return pair_batch_reserve_smem(accum, smem_bytes, max_rows);
   return with_tile_batch(mode, accum, smem_bytes, max_rows, cs, [&](auto fn) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem_bytes);
@@ -1708,6 +1625,8 @@ cudaError_t launch_tile_batch(int mode, int accum, const BatchArgs& b,
                               int smem_bytes, int max_rows, int cs, int sm_count,
                               cudaStream_t st) {
   if (n_items <= 0) return cudaSuccess;
+  if (mode == STRIP_MODE_CPU && cs == kColumnStride)
+    return launch_pair_batch(accum, b, items, n_items, counter, smem_bytes, max_rows, sm_count, st);
   const bool wide = smem_bytes > kNarrowSmemBytes;
   auto pick = [&](auto fn) -> cudaError_t {
     const int grid = std::min(n_items, sm_count * (wide ? 1 : 2));
@@ -1779,9 +1698,10 @@ cudaError_t launch_update(float* rho, double* acc, int64_t n_pix, double scale,
 cudaError_t launch_item_order(const ScannerF& s, const Tiling& t, const WorkItem* items,
                               int n_items, const float* zu, const float* zd, const float* dl,
                               const int64_t* perm, float* ozu, float* ozd, float* odl,
-                              int64_t* operm, cudaStream_t st) {
+                              int64_t* operm, EventPack* packs, cudaStream_t st) {
   if (n_items <= 0) return cudaSuccess;
-  k_item_order<<<n_items, 256, 0, st>>>(s, t, items, zu, zd, dl, perm, ozu, ozd, odl, operm);
+  k_item_order<<<n_items, 256, 0, st>>>(s, t, items, zu, zd, dl, perm, ozu, ozd, odl, operm,
+                                        packs);
   return cudaGetLastError();
 }
 

@@ -105,11 +105,7 @@ KernelF make_kernel(double sigma_z, double sigma_dl, float pw) {
   return k;
 }
 
-// The kernel constants per kc^2, so that rsqrt gives kc / sqrt(a'Sa); and with
-// d = log2 of the rounded q over the true one, pixel j of a run of l + 1
-// carries d j (j - 1) / 2: K0 takes 2^(d (l^2 / 8 - w)) and R0 2^(d (1 - l) / 2),
-// which leaves d ((j - l / 2)^2 / 2 - w), w = sigma_z^2 / 4 its mean over the
-// Gaussian (pixels).
+// The kernel constants per kc^2, so that rsqrt gives kc / sqrt(a'Sa).
 PairConst make_pair_const(const ScannerF& s, const KernelF& k) {
   PairConst c;
   c.nzero = -0.0f;
@@ -124,19 +120,15 @@ PairConst make_pair_const(const ScannerF& s, const KernelF& k) {
   c.cd = -2.0f * kLog2e * k.ipsdl;
   c.c1 = k.c1;
   c.r1 = k.r1;
-  c.q = k.q;
-  const double d = std::log2((double)k.q) - 2.0 * (double)k.c1 * s.pw * s.pw;
-  c.r0 = (float)((double)k.c1 * s.pw * s.pw + 0.5 * d);
-  c.dh = (float)(-0.5 * d);
-  c.d8 = (float)(0.125 * d);
-  c.d0 = (float)(-0.25 * d / ((double)k.ipsz * s.pw * s.pw));
+  c.r0 = k.r0;
+  c.qm1 = (float)std::expm1(2.0 * M_LN2 * (double)k.c1 * s.pw * s.pw);
   return c;
 }
 
 bool pair_const_ok(const PairConst& c) {
   auto in = [](float v, float lo, float hi) { return v > lo && v < hi; };
   return in(c.na4, 1e-25f, 1e25f) && in(c.na2, 1e-25f, 1e25f) && in(c.nb4, 1e-25f, 1e25f) &&
-         in(c.q, 1e-6f, 2.0f) && in(c.c9, 1e-25f, 1e25f) && std::isfinite(c.d0);
+         in(c.qm1, -0.999999f, 0.0f) && in(c.c9, 1e-25f, 1e25f);
 }
 
 }  // namespace stripmlem

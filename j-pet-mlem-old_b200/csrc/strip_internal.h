@@ -112,8 +112,7 @@ struct PairConst {
   float c9, nk4;        // hw^2 = c9 + nk4 sec^2 dy^2, in pixels^2
   float na4, na2, nb4;  // a'Sa / kc^2 = (na4 sec^4 + na2 sec^2 tan^2) yp^2 + nb4 sec^4
   float cd, c1;         // log2 E = c1 t^2 + cd sec^2 dy^2
-  float r1, r0, q;      // ratio 2^(r1 t + r0), ratio of ratios
-  float d8, d0, dh;     // centring of q's rounding error (make_pair_const)
+  float r1, r0, qm1;    // ratio 2^(r1 t + r0), ratio of ratios less one
 };
 // Whether the row-pair kernels can take the kernel's constants.
 bool pair_const_ok(const PairConst& c);

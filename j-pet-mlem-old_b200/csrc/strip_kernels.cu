@@ -2,8 +2,8 @@
 //
 //   k_event_boxes / k_bin_keys / k_bin_scatter   one-time binning of the events
 //       into image tiles (events are iteration-invariant, so this is paid once)
-//   k_tile      the tile kernel (row-major windows, the AnalyticKernel and the
-//       sigma gradient; the GaussianKernel over column-major windows, the
+//   k_tile      the tile kernel (row-major windows and the
+//       AnalyticKernel; the GaussianKernel over column-major windows, the
 //       common case, is strip_pairs.cu's): one CTA per (tile, event chunk) work item.  The
 //       tile's window of the image (tile + halo) is staged in shared memory
 //       next to a shared-memory backprojection accumulator.  A warp takes one
@@ -1461,10 +1461,10 @@ int grid_for(int64_t n, int per_block = kThreads, int cap = 148 * 16) {
 
 constexpr int kSetsCap = 64;
 
-// Column-major windows reach this file's kernels for the AnalyticKernel and
-// the sigma gradient only (the others: launch_pair_tile).
+// Column-major windows reach this file's kernels for the AnalyticKernel only
+// (the GaussianKernel: launch_pair_tile).
 template <int OP, int MODE>
-constexpr bool column_major() { return MODE != STRIP_MODE_CPU || OP == OP_GRAD; }
+constexpr bool column_major() { return MODE != STRIP_MODE_CPU; }
 
 template <int OP, int MODE, int ACC, int LPE, int CS>
 cudaError_t launch_tile_cs(const LaunchArgs& a, cudaStream_t st) {
@@ -1535,7 +1535,7 @@ int tile_column_stride(int WXmax, int WYmax, int budget) {
 cudaError_t launch_tile(int op, int mode, int accum, const LaunchArgs& a,
                         cudaStream_t st) {
   if (a.n_items <= 0) return cudaSuccess;
-  if (mode == STRIP_MODE_CPU && a.t.cs == kColumnStride && op != OP_GRAD)
+  if (mode == STRIP_MODE_CPU && a.t.cs == kColumnStride)
     return launch_pair_tile(op, accum, a, st);
   switch (op) {
     case OP_MLEM:

@@ -1,5 +1,5 @@
 // The tile kernels of the GaussianKernel over column-major windows (MLEM,
-// forward, adjoint): row pairs in packed f32x2 arithmetic.
+// forward, adjoint, sigma gradient): row pairs in packed f32x2 arithmetic.
 //
 // An event is worked on by a group of LPE lanes (8 or 16: four or two events
 // per warp).  Its box rows are paired from the middle out -- rows mid + k and
@@ -21,10 +21,10 @@
 // written as fma(a, b, -0) with a -0 that the compiler cannot see
 // (PairConst::nzero): a * b rounded once, whatever follows.
 //
-// Accuracy.  q (the ratio of neighbouring ratios) is a rounded constant, and
-// its relative error d enters pixel j of a run as d j (j - 1) / 2.  K0 and R0
-// take the correction that turns this into d (j - c)^2 / 2 less its mean, c
-// the run's middle pixel: as if the walk started there.
+// Accuracy.  q (the ratio of neighbouring ratios) would enter pixel j of a run
+// with its rounding error times j (j - 1) / 2.  The ratios advance by
+// R <- R + R (q - 1), one fused operation with q - 1 rounded: the error is
+// smaller by |q - 1| (0.08 at sigma_z = 5 pixels).
 //
 // Backprojection window: unsigned 32-bit fixed point as in strip_kernels.cu
 // (fixed_shift and the unweighted windows of strip_internal.h).  An addend
@@ -67,6 +67,7 @@ struct PairEvent {
   float tan, tanp, x0;   // tan, tan / pw, centre column
   float nk4;             // hw^2 = c9 + nk4 dy^2 (pixels^2)
   float na, nb, cd;      // GaussEvent, norm in units of kc^2
+  float ng;              // its ipsdl ar^2 = ng yp^2
   float cmin, cend;      // box columns [cmin, cend)
   float fm;              // row of pair 0's lower row (mid), as float
   int n_a, n_b;          // rows of the two sides: pairs k < n_a, k < n_b
@@ -97,7 +98,8 @@ __device__ __forceinline__ PairEvent pair_event(const ScannerF& s, const PairCon
   e.x0 = (m.z - s.tl_z_half_w) * s.inv_pw;
   const float s2 = m.sec * m.sec, s4 = s2 * s2;
   e.nk4 = s2 * c.nk4;
-  e.na = c.na4 * s4 + c.na2 * s2 * tt;
+  e.ng = c.na2 * s2 * tt;
+  e.na = fmaf(c.na4, s4, e.ng);
   e.nb = c.nb4 * s4;
   e.cd = c.cd * s2;
   return e;
@@ -109,9 +111,11 @@ __device__ __forceinline__ PairEvent pair_event(const ScannerF& s, const PairCon
 struct PairRow {
   float2 K0, R0;
   unsigned run;
+  float2 t, g, e2;  // sigma gradient: first t, arr / a'Sa, log2 of the row's exp
 };
 
-// Pair k of the event (k_f = k), f32x2 = (row mid + k, row mid - 1 - k).
+// Pair k of the event, f32x2 = (row mid + k, row mid - 1 - k).
+template <bool GRAD = false>
 __device__ __forceinline__ PairRow pair_row(const ScannerF& s, const PairConst& c,
                                             const PairEvent& e, int k, float mw) {
   const float kf = (float)k;
@@ -151,18 +155,22 @@ __device__ __forceinline__ PairRow pair_row(const ScannerF& s, const PairConst& 
   const unsigned ra = len.x >= 1.0f && k < e.n_a ? __float_as_uint(bits.x) : 0u;
   const unsigned rb = len.y >= 1.0f && k < e.n_b ? __float_as_uint(bits.y) : 0u;
   r.run = __byte_perm(ra, rb, 0x5410);
-  // kernel constants (GaussEvent::row) with q's error centred on the run
+  // kernel constants (GaussEvent::row)
   const float2 t0 = __fadd2_rn(__ffma2_rn(lo, dup(s.pw), dup(s.tl_z_half_w)), dup(e.nz));
   const float2 t = __ffma2_rn(dy, dup(-e.tan), t0);
   const float2 yp = __fadd2_rn(dy, dup(-e.ny));
   const float2 norm = __ffma2_rn(dup(e.na), __fmul2_rn(yp, yp), dup(e.nb));
-  const float2 l1 = __fadd2_rn(len, dup(-1.0f));
-  const float2 fix = __ffma2_rn(__fmul2_rn(l1, dup(c.d8)), l1, dup(c.d0));
-  const float2 arg = __ffma2_rn(__fmul2_rn(dup(c.c1), t), t, __ffma2_rn(dup(e.cd), dd, fix));
-  const float2 ar = __ffma2_rn(t, dup(c.r1), __ffma2_rn(l1, dup(c.dh), dup(c.r0)));
+  const float2 arg = __ffma2_rn(__fmul2_rn(dup(c.c1), t), t, __fmul2_rn(dup(e.cd), dd));
+  const float2 ar = __ffma2_rn(t, dup(c.r1), dup(c.r0));
   r.K0 = __fmul2_rn(make_float2(rsqrt_approx(norm.x), rsqrt_approx(norm.y)),
                     make_float2(ex2_approx(arg.x), ex2_approx(arg.y)));
   r.R0 = make_float2(ex2_approx(ar.x), ex2_approx(ar.y));
+  if constexpr (GRAD) {
+    r.t = t;
+    r.g = __fmul2_rn(__fmul2_rn(yp, yp), dup(e.ng));
+    r.g = __fmul2_rn(r.g, make_float2(rcp_approx(norm.x), rcp_approx(norm.y)));
+    r.e2 = __fmul2_rn(dup(e.cd), dd);
+  }
   return r;
 }
 
@@ -195,7 +203,7 @@ __device__ __forceinline__ float pair_sum(float2 P, float2 S, float2 Q, PairWalk
   for (int j = w.n; j > 0; --j, w.a += kColB, w.b += kColB) {
     A = __ffma2_rn(P, make_float2(lds32(w.a), lds32(w.b)), A);
     P = __fmul2_rn(P, S);
-    S = __fmul2_rn(S, Q);
+    S = __ffma2_rn(S, Q, S);
   }
   __syncwarp();
   float sum = A.x + A.y;
@@ -207,13 +215,59 @@ __device__ __forceinline__ float pair_sum(float2 P, float2 S, float2 Q, PairWalk
 #pragma unroll 1
     for (int j = w.m - 1; j > 0; --j) {
       x *= r;
-      r *= Q.x;
+      r = fmaf(r, Q.x, r);
       p += kColB;
       sum = fmaf(x, lds32(p), sum);
     }
     __syncwarp();
   }
   return sum;
+}
+
+// Sums of K w and K w t^2 over the pair's runs (the sigma gradient); t: the
+// distances of the runs' first pixels from the rows' centres.  2e6 events at
+// 400 x 400, sigma_z 8, sigma_dl 30 mm: 6.2 ms with one event per warp, one
+// row per lane and two global binary64 reductions per event on the same two
+// words; 3.0 ms here, with the sums kept in the lanes over the item's events.
+__device__ __forceinline__ void pair_moments(float2 P, float2 S, float2 Q, float2 t, float pw,
+                                             PairWalk w, float2& s0, float2& s2) {
+  s0 = s2 = make_float2(0.0f, 0.0f);
+  const float2 dt = dup(pw), t0 = t;
+  float2 at = make_float2(0.0f, 0.0f);  // steps taken
+#pragma unroll kUnroll
+  for (int j = w.n; j > 0; --j, w.a += kColB, w.b += kColB) {
+    const float2 x = __fmul2_rn(P, make_float2(lds32(w.a), lds32(w.b)));
+    s0 = __fadd2_rn(s0, x);
+    s2 = __ffma2_rn(__fmul2_rn(x, t), t, s2);
+    at = __fadd2_rn(at, dup(1.0f));
+    t = __ffma2_rn(at, dt, t0);
+    P = __fmul2_rn(P, S);
+    S = __ffma2_rn(S, Q, S);
+  }
+  __syncwarp();
+  if (__any_sync(kFull, w.m > 0)) {
+    uint32_t p = w.long_a ? w.a : w.b;
+    float x = w.long_a ? P.x : P.y, r = w.long_a ? S.x : S.y, u = w.long_a ? t.x : t.y;
+    float a0 = 0.0f, a2 = 0.0f;
+#pragma unroll 1
+    for (int j = w.m; j > 0; --j) {
+      const float v = x * lds32(p);
+      a0 += v;
+      a2 = fmaf(v * u, u, a2);
+      u += pw;
+      x *= r;
+      r = fmaf(r, Q.x, r);
+      p += kColB;
+    }
+    if (w.long_a) {
+      s0.x += a0;
+      s2.x += a2;
+    } else {
+      s0.y += a0;
+      s2.y += a2;
+    }
+    __syncwarp();
+  }
 }
 
 // How the backprojection turns a value into window units: K (times the image)
@@ -249,7 +303,7 @@ __device__ __forceinline__ void pair_scatter(float2 P, float2 S, float2 Q, PairW
       red_shared_add(w.b, __float2uint_rn(x.y));
     }
     P = __fmul2_rn(P, S);
-    S = __fmul2_rn(S, Q);
+    S = __ffma2_rn(S, Q, S);
   }
   __syncwarp();
   auto put = [&](uint32_t p, float x) {  // one pixel
@@ -267,7 +321,7 @@ __device__ __forceinline__ void pair_scatter(float2 P, float2 S, float2 Q, PairW
 #pragma unroll 1
     for (int j = w.m - 1; j > 0; --j) {
       x *= r;
-      r *= Q.x;
+      r = fmaf(r, Q.x, r);
       p += kColB;
       put(p, x);
     }
@@ -289,11 +343,12 @@ struct PairWin {
 template <int OP, int ACC, int LPE, int NB, bool WEIGHTED, int ADD>
 __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& it,
                                           const PairWin& win, int lane, int grab,
-                                          int* next_group, const unsigned* only) {
+                                          int* next_group, const unsigned* only,
+                                          double* grad = nullptr) {
   constexpr int kPer = 32 / LPE;
   constexpr int kBlocks = OP == OP_MLEM ? NB : 1;  // kept for pass 2
   const int grp = lane / LPE, sub = lane & (LPE - 1);
-  const float2 Q = dup(a.pc.q);
+  const float2 Q = dup(a.pc.qm1);
   const float mw = 8388608.0f - (float)win.wx0;
   float rsum = 0.0f;
   for (;;) {
@@ -324,6 +379,30 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
           pair_scatter<ADD>(__fmul2_rn(r.K0, dup(wf)), r.R0, Q,
                                    PairWalk(r.run, win.acc + ra + 4u * LPE * b,
                                             win.acc + rb - 4u * LPE * b), 0u);
+        }
+        continue;
+      }
+      if constexpr (OP == OP_GRAD) {
+        // d log K / d sigma (GaussGradRow): with g = ipsdl ar^2 / a'Sa and
+        // brr = -2 ln 2 e2, sigma_z: -1 - g + 2 ipsz t^2, sigma_dl: g + brr - 1.
+        // The lane adds up its rows of all its events in binary64.
+        const double w = has ? a.w_in[a.perm[it.begin + j]] : 0.0;
+        if (!__any_sync(kFull, w != 0.0)) continue;
+        for (int b = 0; b < nb; ++b) {
+          PairRow r = pair_row<true>(a.s, a.pc, e, LPE * b + sub, mw);
+          if (w == 0.0) r.run = 0u;
+          float2 s0, s2;
+          pair_moments(r.K0, r.R0, Q, r.t, a.s.pw,
+                       PairWalk(r.run, win.w + ra + 4u * LPE * b, win.w + rb - 4u * LPE * b), s0,
+                       s2);
+          auto row = [&](float s0, float s2, float g, float e2) {
+            if (s0 != 0.0f) {  // rows without pixels have any g and e2
+              grad[0] += w * (double)fmaf(-1.0f - g, s0, 2.0f * a.k.ipsz * s2);
+              grad[1] += w * (double)((fmaf(-1.3862943611198906f, e2, g) - 1.0f) * s0);
+            }
+          };
+          row(s0.x, s2.x, r.g.x, r.e2.x);
+          row(s0.y, s2.y, r.g.y, r.e2.y);
         }
         continue;
       }
@@ -402,7 +481,7 @@ template <int OP, int ACC, int LPE, int NB>
 __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkItem it, int index,
                                                char* smem_raw, int* s_next_group) {
   constexpr int CS = kColumnStride;
-  constexpr bool kReads = OP != OP_ADJOINT, kWrites = OP != OP_FORWARD;
+  constexpr bool kReads = OP != OP_ADJOINT, kWrites = OP == OP_MLEM || OP == OP_ADJOINT;
   int wx0, wy0, wx1, wy1;
   tile_window(a.t, a.s.n_z, a.s.n_y, it.tile, wx0, wy0, wx1, wy1);
   const int wxn = wx1 - wx0, wyn = wy1 - wy0;
@@ -461,7 +540,20 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
       if (v != 0.0) atomicAdd(a.acc + (int64_t)(wy0 + r) * a.s.n_z + wx0 + c, v);
     });
   };
-  if constexpr (OP == OP_FORWARD) {
+  if constexpr (OP == OP_GRAD) {
+    double grad[2] = {0.0, 0.0};
+    pair_item<OP, ACC, LPE, NB, false, kAddSigned>(a, it, win, lane, grab, s_next_group, nullptr,
+                                                   grad);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      grad[0] += __shfl_xor_sync(kFull, grad[0], o);
+      grad[1] += __shfl_xor_sync(kFull, grad[1], o);
+    }
+    if (lane == 0) {
+      atomicAdd(a.grad_out, grad[0] / a.sz);
+      atomicAdd(a.grad_out + 1, grad[1] / a.sdl);
+    }
+  } else if constexpr (OP == OP_FORWARD) {
     pair_item<OP, ACC, LPE, NB, false, kAddSigned>(a, it, win, lane, grab, s_next_group, nullptr);
   } else if constexpr (OP == OP_ADJOINT) {
     // addends below 2^22 (adjoint_shift); without negative weights the
@@ -651,6 +743,8 @@ cudaError_t launch_pair_tile(int op, int accum, const LaunchArgs& a, cudaStream_
       return launch_pair_op<OP_FORWARD>(accum, a, st);
     case OP_ADJOINT:  // no per-event sums: one form
       return launch_pair_t<OP_ADJOINT, STRIP_ACCUM_FP32>(a, st);
+    case OP_GRAD:
+      return launch_pair_t<OP_GRAD, STRIP_ACCUM_FP32>(a, st);
     default:
       return cudaErrorInvalidValue;
   }

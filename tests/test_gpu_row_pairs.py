@@ -132,3 +132,27 @@ def test_batch_of_both_lane_layouts():
     finally:
         for rec in recs:
             rec.close()
+
+
+@pytest.mark.parametrize("case", CASES)
+@pytest.mark.parametrize("n", [1, 6_001])
+def test_sigma_gradient(case, n):
+    import stripmlem as sm
+    R, L, n_y, n_z, p, s_z, s_dl = case
+    g = orc.geometry(R, L, n_y, n_z, p, p, s_z, s_dl)
+    ev = events(case, n, 9)
+    if n == 1:
+        ev = [np.float32([v]) for v in (0.1 * p, -0.2 * p, 0.3 * p)]
+    r = np.random.default_rng(10)
+    rho = r.lognormal(0.0, 0.5, (n_y, n_z)).astype(np.float32)
+    w = np.where(r.random(n) < 0.1, 0.0, r.uniform(-0.5, 2.0, n)) if n > 1 else np.ones(1)
+    with sm.Reconstruction(sm.Scanner(R, L, n_y, n_z, p, p, s_z, s_dl)) as rec:
+        rec.set_events(*ev)
+        got = rec.grad_sigma(rho, w, 0.9 * s_z, 0.95 * s_dl)
+    o = orc.grad_sigma_f64(g, *ev, rho, w, 0.9 * s_z, 0.95 * s_dl)
+    # a row's derivative is a difference of terms of a few times its value, and
+    # the events' cancel in the sum: bounded by the sum of y |w| / sigma
+    y = orc.forward_f64(g, *ev, rho, 0.9 * s_z, 0.95 * s_dl)
+    scale = np.dot(np.abs(w), y)
+    assert abs(got[0] - o[0]) < IMAGE_TOL * scale / s_z
+    assert abs(got[1] - o[1]) < IMAGE_TOL * scale / s_dl

@@ -31,9 +31,10 @@ using namespace stripmlem;
 
 // Windows up to this size let two CTAs share an SM.
 constexpr int kNarrowSmem = kNarrowSmemBytes;
-// Work-item classes: narrow / wide windows, row-major / column-major.
-constexpr int kClasses = 4;
-inline int class_stride(int c) { return (c & 2) ? kColumnStride : 0; }
+// Work-item classes: narrow / wide windows, row-major / column-major of either
+// stride.
+constexpr int kClasses = 6;
+inline int class_stride(int c) { return c < 2 ? 0 : c < 4 ? kColumnStride : kTallStride; }
 // Members with at least this many work items per SM get a tile launch of
 // their own (k_tile, arguments in constant parameter space) instead of
 // joining the persistent launch, whose per-member arguments are indexed at
@@ -63,9 +64,9 @@ struct strip_batch {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   BatchArgs* args = nullptr;  // host copy of the kernel parameters (~20 KB)
-  // Work items in four classes: members whose windows fit two CTAs per SM
+  // Work items in six classes: members whose windows fit two CTAs per SM
   // and wide-window members (one CTA per SM), each with row-major or
-  // column-major windows (class = wide + 2 * column-major).  Each class is one
+  // column-major windows of either stride (class_stride).  Each class is one
   // persistent launch, so a wide member does not halve the occupancy of the
   // others.  Class c owns items [cls_begin[c], cls_begin[c] + cls_count[c]).
   BatchItem* d_items = nullptr;
@@ -213,7 +214,8 @@ int strip_batch_create(strip_ctx* const* members, int n_members, int mode,
     b->args->member[m] = ctx_mlem_args(c, mode);
     const bool own_launch =
         b->args->member[m].n_items >= STRIP_BATCH_SPLIT_PER_SM * b->sm_count;
-    const int cls = (c->t.smem_bytes > kNarrowSmem) + (c->t.cs != 0 ? 2 : 0);
+    const int cls = (c->t.smem_bytes > kNarrowSmem) +
+                    (c->t.cs == 0 ? 0 : c->t.cs == kColumnStride ? 2 : 4);
     b->cls_smem[cls] = std::max(b->cls_smem[cls], c->t.smem_bytes);
     b->cls_rows[cls] = std::max(b->cls_rows[cls], c->t.max_rows);
     b->n_events += c->n_events;

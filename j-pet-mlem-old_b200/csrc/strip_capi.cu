@@ -213,8 +213,22 @@ Tiling choose_tiling(const strip_ctx* ctx, int max_w, int max_h) {
       ctx->s.min_closed_hw == 0.0f &&
       pair_const_ok(make_pair_const(
           ctx->s, make_kernel(ctx->g.sigma_z, ctx->g.sigma_dl, ctx->s.pw)));
-  t.cs = pairs ? tile_column_stride(t.WXmax, t.WYmax, budget) : 0;
-  if (t.cs) t.smem_bytes = 2 * t.WXmax * t.cs * 4;
+  auto column_bytes = [&](int cs) { return 2 * t.WXmax * cs * 4; };
+  if (pairs && t.WYmax <= kColumnStride && column_bytes(kColumnStride) <= budget) {
+    t.cs = kColumnStride;
+    t.smem_bytes = column_bytes(kColumnStride);
+  } else if (pairs && max_h > kPairRows8 && max_h <= kPairRows16 &&
+             2 * t.HY + 16 <= kTallStride && column_bytes(kTallStride) <= budget) {
+    // Tall boxes: the tile's rows cut to what the tall stride leaves beside
+    // the halos (28 or more at 128 rows).  The row-major form stays possible
+    // for the kernels that take it.  Around smaller boxes such windows come
+    // of large tiles; those stay row-major.  (126-row boxes, 4e5 events, 300 x
+    // 437 pixels of 1 mm: five iterations 25.6 ms row-major, 14.2 ms here.)
+    t.cs = kTallStride;
+    t.TY = std::min(t.TY, kTallStride - 2 * t.HY);
+    t.WYmax = std::min(n_y, t.TY + 2 * t.HY);
+    t.smem_bytes = std::max(tile_smem_bytes(t.WYmax, t.WS), column_bytes(kTallStride));
+  }
   t.ntx = (n_z + t.TX - 1) / t.TX;
   t.nty = (n_y + t.TY - 1) / t.TY;
   t.n_tiles = t.ntx * t.nty;

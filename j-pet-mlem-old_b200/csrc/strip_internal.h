@@ -64,10 +64,16 @@ struct Tiling {
   int WXmax, WYmax, WS;
   int smem_bytes;  // the two shared-memory windows
   int max_rows;    // the most box rows of any event (the kernels' lane layout)
-  int cs;          // window column stride: kColumnStride (column-major) or 0
+  int cs;          // window column stride (column-major), or 0 (row-major)
 };
-// Column stride of column-major tile windows (words; a multiple of 32).
-constexpr int kColumnStride = 128;
+// Column strides of column-major tile windows (words; multiples of 32): of
+// windows up to 128 rows high, and of the taller ones that boxes of 81 to 128
+// rows need, which the row-pair kernels alone take (others read such a
+// tiling's windows row-major).
+constexpr int kColumnStride = 128, kTallStride = 160;
+// The most box rows of the row-pair kernels' lane layouts (8 and 16 lanes an
+// event).
+constexpr int kPairRows8 = 80, kPairRows16 = 128;
 
 __host__ __device__ inline void tile_window(const Tiling& t, int n_z, int n_y,
                                             int tile, int& wx0, int& wy0,
@@ -185,7 +191,6 @@ KernelF make_kernel(double sigma_z, double sigma_dl, float pw);
 
 // ---- launchers (strip_kernels.cu) ----------------------------------------
 int tile_smem_bytes(int WYmax, int WS);
-int tile_column_stride(int WXmax, int WYmax, int budget);
 cudaError_t launch_event_boxes(const ScannerF& s, const float* zu,
                                const float* zd, const float* dl, int64_t n,
                                int4* boxes, int* max_wh, unsigned long long* n_empty,
@@ -211,9 +216,9 @@ cudaError_t launch_item_order(const ScannerF& s, const Tiling& t, const WorkItem
                               int64_t* operm, EventPack* packs, cudaStream_t st);
 // GaussianKernel over column-major windows (strip_pairs.cu).
 cudaError_t launch_pair_tile(int op, int accum, const LaunchArgs& a, cudaStream_t st);
-cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows);
+cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int cs);
 cudaError_t launch_pair_batch(int accum, const BatchArgs& b, const BatchItem* items, int n_items,
-                              int* counter, int smem_bytes, int max_rows, int sm_count,
+                              int* counter, int smem_bytes, int max_rows, int cs, int sm_count,
                               cudaStream_t st);
 cudaError_t launch_global(int op, int mode, int accum, const LaunchArgs& a,
                           cudaStream_t st);

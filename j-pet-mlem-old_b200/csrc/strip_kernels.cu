@@ -42,10 +42,6 @@ constexpr int kWarps = kThreads / 32;
 #define STRIP_TILE_THREADS 512
 #endif
 constexpr int kTileThreads = STRIP_TILE_THREADS;
-// Column-major tile windows where they fit (tile_column_stride).
-#ifndef STRIP_COLUMN_MAJOR
-#define STRIP_COLUMN_MAJOR 1
-#endif
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -1524,18 +1520,10 @@ cudaError_t launch_global_t(const LaunchArgs& a, cudaStream_t st) {
 // Two windows (the image and the accumulator) of WYmax rows of stride WS.
 int tile_smem_bytes(int WYmax, int WS) { return 2 * WYmax * WS * 4; }
 
-// The column stride of a tiling's windows: kColumnStride (column-major) when
-// the windows are at most that many rows high and their column-major form
-// fits `budget` bytes, else 0 (row-major).
-int tile_column_stride(int WXmax, int WYmax, int budget) {
-  if (!STRIP_COLUMN_MAJOR) return 0;
-  return WYmax <= kColumnStride && 2 * WXmax * kColumnStride * 4 <= budget ? kColumnStride : 0;
-}
-
 cudaError_t launch_tile(int op, int mode, int accum, const LaunchArgs& a,
                         cudaStream_t st) {
   if (a.n_items <= 0) return cudaSuccess;
-  if (mode == STRIP_MODE_CPU && a.t.cs == kColumnStride)
+  if (mode == STRIP_MODE_CPU && a.t.cs != 0)
     return launch_pair_tile(op, accum, a, st);
   switch (op) {
     case OP_MLEM:
@@ -1572,7 +1560,7 @@ cudaError_t launch_global(int op, int mode, int accum, const LaunchArgs& a,
 
 template <int THREADS, int CS, class F>
 cudaError_t with_tile_batch_t(int mode, int accum, bool half, F&& pick) {
-  if constexpr (CS == 0)
+  if constexpr (CS == 0)  // column-major members of this mode: launch_pair_batch
   if (mode == STRIP_MODE_CPU) {
     constexpr int H = lanes_per_event<OP_MLEM, STRIP_MODE_CPU>();
     if (half) {
@@ -1612,8 +1600,8 @@ cudaError_t with_tile_batch(int mode, int accum, int smem_bytes, int max_rows, i
 }
 
 cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max_rows, int cs) {
-  if (mode == STRIP_MODE_CPU && cs == kColumnStride)
-    return pair_batch_reserve_smem(accum, smem_bytes, max_rows);
+  if (mode == STRIP_MODE_CPU && cs != 0)
+    return pair_batch_reserve_smem(accum, smem_bytes, max_rows, cs);
   return with_tile_batch(mode, accum, smem_bytes, max_rows, cs, [&](auto fn) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem_bytes);
@@ -1625,8 +1613,9 @@ cudaError_t launch_tile_batch(int mode, int accum, const BatchArgs& b,
                               int smem_bytes, int max_rows, int cs, int sm_count,
                               cudaStream_t st) {
   if (n_items <= 0) return cudaSuccess;
-  if (mode == STRIP_MODE_CPU && cs == kColumnStride)
-    return launch_pair_batch(accum, b, items, n_items, counter, smem_bytes, max_rows, sm_count, st);
+  if (mode == STRIP_MODE_CPU && cs != 0)
+    return launch_pair_batch(accum, b, items, n_items, counter, smem_bytes, max_rows, cs, sm_count,
+                             st);
   const bool wide = smem_bytes > kNarrowSmemBytes;
   auto pick = [&](auto fn) -> cudaError_t {
     const int grid = std::min(n_items, sm_count * (wide ? 1 : 2));

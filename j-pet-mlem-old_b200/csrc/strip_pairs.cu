@@ -52,7 +52,6 @@ constexpr int kPairWide = 2 * kPairThreads;  // one CTA per SM
 // four; eight everywhere 3.97, one 4.38).
 constexpr int kUnroll = 4;
 __host__ __device__ constexpr int sum_unroll(int op) { return op == OP_MLEM ? 2 : kUnroll; }
-constexpr uint32_t kColB = 4u * kColumnStride;  // bytes between columns
 
 __device__ __forceinline__ float2 dup(float x) { return make_float2(x, x); }
 // a * b, rounded, never fused with what follows
@@ -177,7 +176,9 @@ __device__ __forceinline__ PairRow pair_row(const ScannerF& s, const PairConst& 
 // The two runs of a pair as shared-space addresses of their first pixels
 // (relative to a window base) and lengths: n steps together, then m of the
 // longer one (a if long_a).
+template <int CS>
 struct PairWalk {
+  static constexpr uint32_t kColB = 4u * CS;  // bytes between columns
   uint32_t a, b;
   int n, m;
   bool long_a;
@@ -196,8 +197,9 @@ struct PairWalk {
 // has them -- tips and clipped boxes -- the rest.
 
 // Sum of K w over the pair's runs.
-template <int UNROLL>
-__device__ __forceinline__ float pair_sum(float2 P, float2 S, float2 Q, PairWalk w) {
+template <int UNROLL, int CS>
+__device__ __forceinline__ float pair_sum(float2 P, float2 S, float2 Q, PairWalk<CS> w) {
+  constexpr uint32_t kColB = PairWalk<CS>::kColB;
   float2 A = make_float2(0.0f, 0.0f);
 #pragma unroll UNROLL
   for (int j = w.n; j > 0; --j, w.a += kColB, w.b += kColB) {
@@ -229,8 +231,10 @@ __device__ __forceinline__ float pair_sum(float2 P, float2 S, float2 Q, PairWalk
 // 400 x 400, sigma_z 8, sigma_dl 30 mm: 6.2 ms with one event per warp, one
 // row per lane and two global binary64 reductions per event on the same two
 // words; 3.0 ms here, with the sums kept in the lanes over the item's events.
+template <int CS>
 __device__ __forceinline__ void pair_moments(float2 P, float2 S, float2 Q, float2 t, float pw,
-                                             PairWalk w, float2& s0, float2& s2) {
+                                             PairWalk<CS> w, float2& s0, float2& s2) {
+  constexpr uint32_t kColB = PairWalk<CS>::kColB;
   s0 = s2 = make_float2(0.0f, 0.0f);
   const float2 dt = dup(pw), t0 = t;
   float2 at = make_float2(0.0f, 0.0f);  // steps taken
@@ -277,9 +281,10 @@ enum { kAddSubnormal, kAddCvt, kAddWeightedSubnormal, kAddWeightedCvt, kAddSigne
 // acc += K (in window units: P carries the event's factor) over the pair's
 // runs; w: addresses in the accumulator window, off: from there to the image
 // window.
-template <int ADD>
-__device__ __forceinline__ void pair_scatter(float2 P, float2 S, float2 Q, PairWalk w,
+template <int ADD, int CS>
+__device__ __forceinline__ void pair_scatter(float2 P, float2 S, float2 Q, PairWalk<CS> w,
                                              uint32_t off) {
+  constexpr uint32_t kColB = PairWalk<CS>::kColB;
   constexpr bool kWeighted = ADD == kAddWeightedSubnormal || ADD == kAddWeightedCvt;
   constexpr bool kSub = ADD == kAddSubnormal || ADD == kAddWeightedSubnormal;
   const float tiny = __uint_as_float(1u);  // 2^-149
@@ -340,7 +345,7 @@ struct PairWin {
 // item's counter.  MLEM: WEIGHTED adds K rho / D, else K / D, with the events
 // that the conversion or the window's budget has no room for marked in
 // s_fb_bits; `only`: the marked events (unmarked as they find room).
-template <int OP, int ACC, int LPE, int NB, bool WEIGHTED, int ADD>
+template <int OP, int ACC, int LPE, int NB, int CS, bool WEIGHTED, int ADD>
 __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& it,
                                           const PairWin& win, int lane, int grab,
                                           int* next_group, const unsigned* only,
@@ -376,8 +381,8 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
         for (int b = 0; b < nb; ++b) {
           PairRow r = pair_row(a.s, a.pc, e, LPE * b + sub, mw);
           if (wf == 0.0f) r.run = 0u;
-          pair_scatter<ADD>(__fmul2_rn(r.K0, dup(wf)), r.R0, Q,
-                                   PairWalk(r.run, win.acc + ra + 4u * LPE * b,
+          pair_scatter<ADD, CS>(__fmul2_rn(r.K0, dup(wf)), r.R0, Q,
+                                   PairWalk<CS>(r.run, win.acc + ra + 4u * LPE * b,
                                             win.acc + rb - 4u * LPE * b), 0u);
         }
         continue;
@@ -392,8 +397,8 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
           PairRow r = pair_row<true>(a.s, a.pc, e, LPE * b + sub, mw);
           if (w == 0.0) r.run = 0u;
           float2 s0, s2;
-          pair_moments(r.K0, r.R0, Q, r.t, a.s.pw,
-                       PairWalk(r.run, win.w + ra + 4u * LPE * b, win.w + rb - 4u * LPE * b), s0,
+          pair_moments<CS>(r.K0, r.R0, Q, r.t, a.s.pw,
+                       PairWalk<CS>(r.run, win.w + ra + 4u * LPE * b, win.w + rb - 4u * LPE * b), s0,
                        s2);
           auto row = [&](float s0, float s2, float g, float e2) {
             if (s0 != 0.0f) {  // rows without pixels have any g and e2
@@ -411,7 +416,7 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
       if constexpr (OP == OP_FORWARD) {
         for (int b = 0; b < nb; ++b) {
           const PairRow r = pair_row(a.s, a.pc, e, LPE * b + sub, mw);
-          sum.add(pair_sum<sum_unroll(OP)>(r.K0, r.R0, Q, PairWalk(r.run, win.w + ra + 4u * LPE * b,
+          sum.add(pair_sum<sum_unroll(OP), CS>(r.K0, r.R0, Q, PairWalk<CS>(r.run, win.w + ra + 4u * LPE * b,
                                                    win.w + rb - 4u * LPE * b)));
         }
       } else {
@@ -419,8 +424,8 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
         for (int b = 0; b < NB; ++b) {
           if (b < nb) {
             rows[b] = pair_row(a.s, a.pc, e, LPE * b + sub, mw);
-            sum.add(pair_sum<sum_unroll(OP)>(rows[b].K0, rows[b].R0, Q,
-                             PairWalk(rows[b].run, win.w + ra + 4u * LPE * b,
+            sum.add(pair_sum<sum_unroll(OP), CS>(rows[b].K0, rows[b].R0, Q,
+                             PairWalk<CS>(rows[b].run, win.w + ra + 4u * LPE * b,
                                       win.w + rb - 4u * LPE * b)));
           }
         }
@@ -464,8 +469,8 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         if (b < nb)
-          pair_scatter<ADD>(__fmul2_rn(rows[b].K0, sc), rows[b].R0, Q,
-                            PairWalk(go ? rows[b].run : 0u, win.acc + ra + 4u * LPE * b,
+          pair_scatter<ADD, CS>(__fmul2_rn(rows[b].K0, sc), rows[b].R0, Q,
+                            PairWalk<CS>(go ? rows[b].run : 0u, win.acc + ra + 4u * LPE * b,
                                      win.acc + rb - 4u * LPE * b),
                             win.w - win.acc);
       }
@@ -477,10 +482,9 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
 // One work item on the whole CTA: stage the window, run the events, flush.
 // `index` is the item's index among the launch's items (its statistic in
 // a.item_hist).  The caller synchronises before the shared memory is reused.
-template <int OP, int ACC, int LPE, int NB>
+template <int OP, int ACC, int LPE, int NB, int CS>
 __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkItem it, int index,
                                                char* smem_raw, int* s_next_group) {
-  constexpr int CS = kColumnStride;
   constexpr bool kReads = OP != OP_ADJOINT, kWrites = OP == OP_MLEM || OP == OP_ADJOINT;
   int wx0, wy0, wx1, wy1;
   tile_window(a.t, a.s.n_z, a.s.n_y, it.tile, wx0, wy0, wx1, wy1);
@@ -542,7 +546,7 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
   };
   if constexpr (OP == OP_GRAD) {
     double grad[2] = {0.0, 0.0};
-    pair_item<OP, ACC, LPE, NB, false, kAddSigned>(a, it, win, lane, grab, s_next_group, nullptr,
+    pair_item<OP, ACC, LPE, NB, CS, false, kAddSigned>(a, it, win, lane, grab, s_next_group, nullptr,
                                                    grad);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -554,7 +558,7 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
       atomicAdd(a.grad_out + 1, grad[1] / a.sdl);
     }
   } else if constexpr (OP == OP_FORWARD) {
-    pair_item<OP, ACC, LPE, NB, false, kAddSigned>(a, it, win, lane, grab, s_next_group, nullptr);
+    pair_item<OP, ACC, LPE, NB, CS, false, kAddSigned>(a, it, win, lane, grab, s_next_group, nullptr);
   } else if constexpr (OP == OP_ADJOINT) {
     // addends below 2^22 (adjoint_shift); without negative weights the
     // subnormal conversion gives the same integers without the subtractions
@@ -562,10 +566,10 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
     const int fshift = adjoint_shift(a, it, lane, &negative);
     win.unit = exp2f((float)fshift);
     if (negative)
-      pair_item<OP, ACC, LPE, NB, false, kAddSigned>(a, it, win, lane, grab, s_next_group,
+      pair_item<OP, ACC, LPE, NB, CS, false, kAddSigned>(a, it, win, lane, grab, s_next_group,
                                                      nullptr);
     else
-      pair_item<OP, ACC, LPE, NB, false, kAddSubnormal>(a, it, win, lane, grab, s_next_group,
+      pair_item<OP, ACC, LPE, NB, CS, false, kAddSubnormal>(a, it, win, lane, grab, s_next_group,
                                                         nullptr);
     __syncthreads();
     flush(fshift, false);
@@ -590,7 +594,7 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
       // again by cvt.rni); smaller items have larger ones
       bool late = false;
       if (it.count >= 512) {
-        pair_item<OP, ACC, LPE, NB, false, kAddSubnormal>(a, it, win, lane, grab, s_next_group,
+        pair_item<OP, ACC, LPE, NB, CS, false, kAddSubnormal>(a, it, win, lane, grab, s_next_group,
                                                           nullptr);
         __syncthreads();
         late = s_fb_n > 0;
@@ -601,7 +605,7 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
         }
       }
       if (it.count < 512 || late)
-        pair_item<OP, ACC, LPE, NB, false, kAddCvt>(a, it, win, lane, grab, s_next_group,
+        pair_item<OP, ACC, LPE, NB, CS, false, kAddCvt>(a, it, win, lane, grab, s_next_group,
                                                     late ? s_fb_bits : nullptr);
       __syncthreads();
       flush(fshift, true);
@@ -621,10 +625,10 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
       win.unit = exp2f((float)fs);
       // K rho / D <= 1: addends up to the unit
       if (fs <= 23)
-        pair_item<OP, ACC, LPE, NB, true, kAddWeightedSubnormal>(a, it, win, lane, grab,
+        pair_item<OP, ACC, LPE, NB, CS, true, kAddWeightedSubnormal>(a, it, win, lane, grab,
                                                                  s_next_group, only);
       else
-        pair_item<OP, ACC, LPE, NB, true, kAddWeightedCvt>(a, it, win, lane, grab, s_next_group,
+        pair_item<OP, ACC, LPE, NB, CS, true, kAddWeightedCvt>(a, it, win, lane, grab, s_next_group,
                                                            only);
       __syncthreads();
       flush(fs, false);
@@ -633,24 +637,27 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
   }
 }
 
-template <int OP, int ACC, int THREADS, int LPE, int NB>
+template <int OP, int ACC, int THREADS, int LPE, int NB, int CS>
 __global__ void __launch_bounds__(THREADS, THREADS == kPairWide ? 1 : 2)
     k_pair_tile(const __grid_constant__ LaunchArgs a) {
   extern __shared__ __align__(16) char smem_raw[];
   __shared__ int s_next_group;
-  pair_tile_item<OP, ACC, LPE, NB>(a, a.items[blockIdx.x], blockIdx.x, smem_raw, &s_next_group);
+  pair_tile_item<OP, ACC, LPE, NB, CS>(a, a.items[blockIdx.x], blockIdx.x, smem_raw, &s_next_group);
 }
 
-// Blocks of row pairs held through both passes: windows are at most 128 rows
-// high, so 5 blocks of 8 pairs (80 rows) or 4 of 16 (128 rows) hold any event.
+// Blocks of row pairs held through both passes: 5 blocks of 8 pairs (80 rows)
+// or 4 of 16 (128 rows).  Boxes of at most 80 rows take 8 lanes an event; the
+// windows of taller ones have the tall column stride where they need it
+// (tile_column_stride).
 constexpr int kBlocks8 = 5, kBlocks16 = 4;
+static_assert(16 * kBlocks8 == kPairRows8 && 32 * kBlocks16 == kPairRows16, "row-pair layouts");
 
-template <int OP, int ACC, int LPE, int NB>
+template <int OP, int ACC, int LPE, int NB, int CS>
 cudaError_t launch_pair_lpe(const LaunchArgs& a, cudaStream_t st) {
   const int smem = a.t.smem_bytes / 2 * (OP == OP_MLEM ? 2 : 1);
   const bool wide = smem > kNarrowSmemBytes;  // one CTA per SM
-  auto fn = wide ? k_pair_tile<OP, ACC, kPairWide, LPE, NB>
-                 : k_pair_tile<OP, ACC, kPairThreads, LPE, NB>;
+  auto fn = wide ? k_pair_tile<OP, ACC, kPairWide, LPE, NB, CS>
+                 : k_pair_tile<OP, ACC, kPairThreads, LPE, NB, CS>;
   cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;
   fn<<<a.n_items, wide ? kPairWide : kPairThreads, smem, st>>>(a);
@@ -659,10 +666,15 @@ cudaError_t launch_pair_lpe(const LaunchArgs& a, cudaStream_t st) {
 
 template <int OP, int ACC>
 cudaError_t launch_pair_t(const LaunchArgs& a, cudaStream_t st) {
+  const bool tall = a.t.cs == kTallStride;
   if constexpr (OP == OP_MLEM) {
-    if (a.t.max_rows > 16 * kBlocks8) return launch_pair_lpe<OP, ACC, 16, kBlocks16>(a, st);
+    if (tall) return launch_pair_lpe<OP, ACC, 16, kBlocks16, kTallStride>(a, st);
+    if (a.t.max_rows > kPairRows8)
+      return launch_pair_lpe<OP, ACC, 16, kBlocks16, kColumnStride>(a, st);
+  } else {
+    if (tall) return launch_pair_lpe<OP, ACC, 8, kBlocks8, kTallStride>(a, st);
   }
-  return launch_pair_lpe<OP, ACC, 8, kBlocks8>(a, st);
+  return launch_pair_lpe<OP, ACC, 8, kBlocks8, kColumnStride>(a, st);
 }
 
 template <int OP>
@@ -679,7 +691,7 @@ namespace {
 // Persistent form over the work items of several reconstructions: a CTA takes
 // item after item from a global counter; item i belongs to member
 // items[i].member, whose arguments live in the kernel's parameter space.
-template <int ACC, int THREADS, int LPE, int NB>
+template <int ACC, int THREADS, int LPE, int NB, int CS>
 __global__ void __launch_bounds__(THREADS, THREADS == kPairWide ? 1 : 2)
     k_pair_batch(const __grid_constant__ BatchArgs b, const BatchItem* items, int n_items,
                  int* counter) {
@@ -692,43 +704,48 @@ __global__ void __launch_bounds__(THREADS, THREADS == kPairWide ? 1 : 2)
     const int i = s_item;
     if (i >= n_items) break;
     const BatchItem bi = items[i];
-    pair_tile_item<OP_MLEM, ACC, LPE, NB>(b.member[bi.member],
+    pair_tile_item<OP_MLEM, ACC, LPE, NB, CS>(b.member[bi.member],
                                           WorkItem{bi.tile, bi.count, bi.begin}, bi.index,
                                           smem_raw, &s_next_group);
     __syncthreads();  // before the next item's window overwrites this one
   }
 }
 
-template <int THREADS, int LPE, int NB, class F>
+template <int THREADS, int LPE, int NB, int CS, class F>
 cudaError_t with_pair_batch_t(int accum, F&& pick) {
-  if (accum == STRIP_ACCUM_FP32) return pick(k_pair_batch<STRIP_ACCUM_FP32, THREADS, LPE, NB>);
-  if (accum == STRIP_ACCUM_FP64) return pick(k_pair_batch<STRIP_ACCUM_FP64, THREADS, LPE, NB>);
-  return pick(k_pair_batch<STRIP_ACCUM_KAHAN, THREADS, LPE, NB>);
+  if (accum == STRIP_ACCUM_FP32) return pick(k_pair_batch<STRIP_ACCUM_FP32, THREADS, LPE, NB, CS>);
+  if (accum == STRIP_ACCUM_FP64) return pick(k_pair_batch<STRIP_ACCUM_FP64, THREADS, LPE, NB, CS>);
+  return pick(k_pair_batch<STRIP_ACCUM_KAHAN, THREADS, LPE, NB, CS>);
+}
+
+template <int LPE, int NB, int CS, class F>
+cudaError_t with_pair_batch_w(int accum, int smem_bytes, F&& pick) {
+  return smem_bytes > kNarrowSmemBytes ? with_pair_batch_t<kPairWide, LPE, NB, CS>(accum, pick)
+                                       : with_pair_batch_t<kPairThreads, LPE, NB, CS>(accum, pick);
 }
 
 template <class F>
-cudaError_t with_pair_batch(int accum, int smem_bytes, int max_rows, F&& pick) {
-  const bool wide = smem_bytes > kNarrowSmemBytes;
-  if (max_rows <= 16 * kBlocks8)
-    return wide ? with_pair_batch_t<kPairWide, 8, kBlocks8>(accum, pick)
-                : with_pair_batch_t<kPairThreads, 8, kBlocks8>(accum, pick);
-  return wide ? with_pair_batch_t<kPairWide, 16, kBlocks16>(accum, pick)
-              : with_pair_batch_t<kPairThreads, 16, kBlocks16>(accum, pick);
+cudaError_t with_pair_batch(int accum, int smem_bytes, int max_rows, int cs, F&& pick) {
+  if (cs == kTallStride)
+    return with_pair_batch_w<16, kBlocks16, kTallStride>(accum, smem_bytes, pick);
+  if (max_rows > kPairRows8)
+    return with_pair_batch_w<16, kBlocks16, kColumnStride>(accum, smem_bytes, pick);
+  return with_pair_batch_w<8, kBlocks8, kColumnStride>(accum, smem_bytes, pick);
 }
 
 }  // namespace
 
-cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows) {
-  return with_pair_batch(accum, smem_bytes, max_rows, [&](auto fn) {
+cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int cs) {
+  return with_pair_batch(accum, smem_bytes, max_rows, cs, [&](auto fn) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   });
 }
 
 cudaError_t launch_pair_batch(int accum, const BatchArgs& b, const BatchItem* items, int n_items,
-                              int* counter, int smem_bytes, int max_rows, int sm_count,
+                              int* counter, int smem_bytes, int max_rows, int cs, int sm_count,
                               cudaStream_t st) {
   const bool wide = smem_bytes > kNarrowSmemBytes;
-  return with_pair_batch(accum, smem_bytes, max_rows, [&](auto fn) -> cudaError_t {
+  return with_pair_batch(accum, smem_bytes, max_rows, cs, [&](auto fn) -> cudaError_t {
     const int grid = std::min(n_items, sm_count * (wide ? 1 : 2));
     fn<<<grid, wide ? kPairWide : kPairThreads, smem_bytes, st>>>(b, items, n_items, counter);
     return cudaGetLastError();

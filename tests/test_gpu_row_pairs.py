@@ -34,6 +34,7 @@ CASES = [
     (400.0, 800.0, 400, 800, 1.0, 5.0, 25.0),    # 76 rows, five blocks
     (100.0, 200.0, 211, 203, 1.0, 4.0, 26.5),    # 80 rows
     (100.0, 200.0, 211, 203, 1.0, 4.0, 27.2),    # 82 rows: 16 lanes an event
+    (150.0, 300.0, 190, 211, 1.0, 6.0, 42.0),    # 126 rows: the tall column stride
     (60.0, 100.0, 111, 97, 1.0, 4.0, 30.0),      # whole image in one window
     (300.0, 500.0, 37, 53, 10.0, 12.0, 30.0),    # boxes of 4 to 10 rows
     (300.0, 500.0, 5, 300, 2.0, 10.0, 42.0),     # a few rows, clipped boxes

@@ -24,7 +24,8 @@
 // Accuracy.  q (the ratio of neighbouring ratios) would enter pixel j of a run
 // with its rounding error times j (j - 1) / 2.  The ratios advance by
 // R <- R + R (q - 1), one fused operation with q - 1 rounded: the error is
-// smaller by |q - 1| (0.08 at sigma_z = 5 pixels).
+// smaller by |q - 1| (0.08 at sigma_z = 5 pixels).  (Not in the sigma
+// gradient, which keeps the one-row kernel's steps.)
 //
 // Backprojection window: unsigned 32-bit fixed point as in strip_kernels.cu
 // (fixed_shift and the unweighted windows of strip_internal.h).  An addend
@@ -66,7 +67,6 @@ struct PairEvent {
   float tan, tanp, x0;   // tan, tan / pw, centre column
   float nk4;             // hw^2 = c9 + nk4 dy^2 (pixels^2)
   float na, nb, cd;      // GaussEvent, norm in units of kc^2
-  float ng;              // its ipsdl ar^2 = ng yp^2
   float cmin, cend;      // box columns [cmin, cend)
   float fm;              // row of pair 0's lower row (mid), as float
   int n_a, n_b;          // rows of the two sides: pairs k < n_a, k < n_b
@@ -97,8 +97,7 @@ __device__ __forceinline__ PairEvent pair_event(const ScannerF& s, const PairCon
   e.x0 = (m.z - s.tl_z_half_w) * s.inv_pw;
   const float s2 = m.sec * m.sec, s4 = s2 * s2;
   e.nk4 = s2 * c.nk4;
-  e.ng = c.na2 * s2 * tt;
-  e.na = fmaf(c.na4, s4, e.ng);
+  e.na = fmaf(c.na4, s4, c.na2 * s2 * tt);
   e.nb = c.nb4 * s4;
   e.cd = c.cd * s2;
   return e;
@@ -110,7 +109,7 @@ __device__ __forceinline__ PairEvent pair_event(const ScannerF& s, const PairCon
 struct PairRow {
   float2 K0, R0;
   unsigned run;
-  float2 t, g, e2;  // sigma gradient: first t, arr / a'Sa, log2 of the row's exp
+  float2 dy, lo;  // sigma gradient: the rows' distances from y, the runs' first columns
 };
 
 // Pair k of the event, f32x2 = (row mid + k, row mid - 1 - k).
@@ -165,10 +164,8 @@ __device__ __forceinline__ PairRow pair_row(const ScannerF& s, const PairConst& 
                     make_float2(ex2_approx(arg.x), ex2_approx(arg.y)));
   r.R0 = make_float2(ex2_approx(ar.x), ex2_approx(ar.y));
   if constexpr (GRAD) {
-    r.t = t;
-    r.g = __fmul2_rn(__fmul2_rn(yp, yp), dup(e.ng));
-    r.g = __fmul2_rn(r.g, make_float2(rcp_approx(norm.x), rcp_approx(norm.y)));
-    r.e2 = __fmul2_rn(dup(e.cd), dd);
+    r.dy = dy;
+    r.lo = lo;
   }
   return r;
 }
@@ -228,9 +225,9 @@ __device__ __forceinline__ float pair_sum(float2 P, float2 S, float2 Q, PairWalk
 
 // Sums of K w and K w t^2 over the pair's runs (the sigma gradient); t: the
 // distances of the runs' first pixels from the rows' centres.  2e6 events at
-// 400 x 400, sigma_z 8, sigma_dl 30 mm: 6.2 ms with one event per warp, one
+// 400 x 400, sigma_z 8, sigma_dl 30 mm: 6.5 ms with one event per warp, one
 // row per lane and two global binary64 reductions per event on the same two
-// words; 3.0 ms here, with the sums kept in the lanes over the item's events.
+// words; 2.7 ms here, with the sums kept in the lanes over the item's events.
 template <int CS>
 __device__ __forceinline__ void pair_moments(float2 P, float2 S, float2 Q, float2 t, float pw,
                                              PairWalk<CS> w, float2& s0, float2& s2) {
@@ -246,7 +243,7 @@ __device__ __forceinline__ void pair_moments(float2 P, float2 S, float2 Q, float
     at = __fadd2_rn(at, dup(1.0f));
     t = __ffma2_rn(at, dt, t0);
     P = __fmul2_rn(P, S);
-    S = __ffma2_rn(S, Q, S);
+    S = __fmul2_rn(S, Q);
   }
   __syncwarp();
   if (__any_sync(kFull, w.m > 0)) {
@@ -260,7 +257,7 @@ __device__ __forceinline__ void pair_moments(float2 P, float2 S, float2 Q, float
       a2 = fmaf(v * u, u, a2);
       u += pw;
       x *= r;
-      r = fmaf(r, Q.x, r);
+      r *= Q.x;
       p += kColB;
     }
     if (w.long_a) {
@@ -388,26 +385,37 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
         continue;
       }
       if constexpr (OP == OP_GRAD) {
-        // d log K / d sigma (GaussGradRow): with g = ipsdl ar^2 / a'Sa and
-        // brr = -2 ln 2 e2, sigma_z: -1 - g + 2 ipsz t^2, sigma_dl: g + brr - 1.
-        // The lane adds up its rows of all its events in binary64.
+        // The lane adds up its rows of all its events in binary64.  A row's
+        // values and steps are the one-row kernel's (grad_event): its sums
+        // cancel to a few hundredths of their terms, so that other roundings
+        // of the same row -- of q above all, 3e-5 at sigma_z of 10 pixels --
+        // would set the two kernels' gradients apart by more than 2e-5.
         const double w = has ? a.w_in[a.perm[it.begin + j]] : 0.0;
         if (!__any_sync(kFull, w != 0.0)) continue;
         for (int b = 0; b < nb; ++b) {
           PairRow r = pair_row<true>(a.s, a.pc, e, LPE * b + sub, mw);
           if (w == 0.0) r.run = 0u;
+          GaussGradRow ga, gb;
+          ga.init(a.k, a.s.R, m.y, m.tan, m.sec, r.dy.x);
+          gb.init(a.k, a.s.R, m.y, m.tan, m.sec, r.dy.y);
+          const float2 t = make_float2(fmaf(r.lo.x, a.s.pw, a.s.tl_z_half_w) - m.z - ga.dytan,
+                                       fmaf(r.lo.y, a.s.pw, a.s.tl_z_half_w) - m.z - gb.dytan);
+          const float2 K0 = make_float2(ex2_approx(fmaf(a.k.c1 * t.x, t.x, ga.c0)),
+                                        ex2_approx(fmaf(a.k.c1 * t.y, t.y, gb.c0)));
+          const float2 R0 = make_float2(ex2_approx(fmaf(a.k.r1, t.x, a.k.r0)),
+                                        ex2_approx(fmaf(a.k.r1, t.y, a.k.r0)));
           float2 s0, s2;
-          pair_moments<CS>(r.K0, r.R0, Q, r.t, a.s.pw,
-                       PairWalk<CS>(r.run, win.w + ra + 4u * LPE * b, win.w + rb - 4u * LPE * b), s0,
-                       s2);
-          auto row = [&](float s0, float s2, float g, float e2) {
-            if (s0 != 0.0f) {  // rows without pixels have any g and e2
-              grad[0] += w * (double)fmaf(-1.0f - g, s0, 2.0f * a.k.ipsz * s2);
-              grad[1] += w * (double)((fmaf(-1.3862943611198906f, e2, g) - 1.0f) * s0);
+          pair_moments<CS>(K0, R0, dup(a.k.q), t, a.s.pw,
+                           PairWalk<CS>(r.run, win.w + ra + 4u * LPE * b,
+                                        win.w + rb - 4u * LPE * b), s0, s2);
+          auto row = [&](const GaussGradRow& g, float s0, float s2) {
+            if (s0 != 0.0f) {  // rows without pixels have any pref, fz and fdl
+              grad[0] += w * (double)(g.pref * fmaf(g.fz, s0, 2.0f * a.k.ipsz * s2));
+              grad[1] += w * (double)(g.pref * g.fdl * s0);
             }
           };
-          row(s0.x, s2.x, r.g.x, r.e2.x);
-          row(s0.y, s2.y, r.g.y, r.e2.y);
+          row(ga, s0.x, s2.x);
+          row(gb, s0.y, s2.y);
         }
         continue;
       }

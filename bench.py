@@ -45,11 +45,11 @@ PHANTOM = [
     (0, 0, 360, 175, 0, 0.2),
 ]
 SEED = 20260101
-# DRAM bytes (read + write) per event of one k_tile pass, from an ncu capture
-# of one launch over this workload's first 2e7 events (dram__bytes_read.sum
-# 244.7 MB + dram__bytes_write.sum 5.1 MB); the traffic grows with the event
-# count.
-TILE_DRAM_BYTES_PER_EVENT = (244.702464e6 + 5.090304e6) / 2e7
+# DRAM bytes (read + write) per event of one k_pair_tile MLEM pass, from an
+# ncu capture of one launch over 2e7 events of this geometry
+# (dram__bytes_read.sum 484.7 MB + dram__bytes_write.sum 2.4 MB: the events'
+# 24-byte packs); the traffic grows with the event count.
+TILE_DRAM_BYTES_PER_EVENT = (484.657152e6 + 2.423040e6) / 2e7
 
 
 def workload_config(n_events, e2e_iters, world=1):

@@ -31,10 +31,9 @@ using namespace stripmlem;
 
 // Windows up to this size let two CTAs share an SM.
 constexpr int kNarrowSmem = kNarrowSmemBytes;
-// Work-item classes: narrow / wide windows, row-major / column-major of either
-// stride.
-constexpr int kClasses = 6;
-inline int class_stride(int c) { return c < 2 ? 0 : c < 4 ? kColumnStride : kTallStride; }
+// Work-item classes: narrow / wide windows of each kind (windows_of).
+constexpr int kClasses = 8;
+inline int class_windows(int c) { return c >> 1; }
 // Members with at least this many work items per SM get a tile launch of
 // their own (k_tile, arguments in constant parameter space) instead of
 // joining the persistent launch, whose per-member arguments are indexed at
@@ -64,9 +63,9 @@ struct strip_batch {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   BatchArgs* args = nullptr;  // host copy of the kernel parameters (~20 KB)
-  // Work items in six classes: members whose windows fit two CTAs per SM
-  // and wide-window members (one CTA per SM), each with row-major or
-  // column-major windows of either stride (class_stride).  Each class is one
+  // Work items in eight classes: members whose windows fit two CTAs per SM
+  // and wide-window members (one CTA per SM), each with windows of the four
+  // kinds (class_windows).  Each class is one
   // persistent launch, so a wide member does not halve the occupancy of the
   // others.  Class c owns items [cls_begin[c], cls_begin[c] + cls_count[c]).
   BatchItem* d_items = nullptr;
@@ -142,7 +141,7 @@ int enqueue_step(strip_batch* b) {
       BCK(launch_tile_batch(b->mode, b->accum, *b->args,
                             b->d_items + b->cls_begin[c], b->cls_count[c],
                             b->d_counter + c, b->cls_smem[c], b->cls_rows[c],
-                            class_stride(c), b->sm_count, b->stream));
+                            class_windows(c), b->sm_count, b->stream));
   for (int s = 0; s < b->n_side; ++s) BCK(cudaStreamWaitEvent(b->stream, b->join[s], 0));
   BatchUpdateArgs u{};
   u.n = (int)b->members.size();
@@ -214,8 +213,8 @@ int strip_batch_create(strip_ctx* const* members, int n_members, int mode,
     b->args->member[m] = ctx_mlem_args(c, mode);
     const bool own_launch =
         b->args->member[m].n_items >= STRIP_BATCH_SPLIT_PER_SM * b->sm_count;
-    const int cls = (c->t.smem_bytes > kNarrowSmem) +
-                    (c->t.cs == 0 ? 0 : c->t.cs == kColumnStride ? 2 : 4);
+    const int cls =
+        (c->t.smem_bytes > kNarrowSmem) + 2 * windows_of(b->args->member[m]);
     b->cls_smem[cls] = std::max(b->cls_smem[cls], c->t.smem_bytes);
     b->cls_rows[cls] = std::max(b->cls_rows[cls], c->t.max_rows);
     b->n_events += c->n_events;
@@ -289,7 +288,7 @@ int strip_batch_create(strip_ctx* const* members, int n_members, int mode,
       for (int c = 0; c < kClasses; ++c)
         if (b->cls_count[c] > 0 &&
             tile_batch_reserve_smem(b->mode, b->accum, b->cls_smem[c], b->cls_rows[c],
-                                    class_stride(c)) != cudaSuccess)
+                                    class_windows(c)) != cudaSuccess)
           attr_ok = false;
       if (!attr_ok ||
           cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {

@@ -125,9 +125,9 @@ PairConst make_pair_const(const ScannerF& s, const KernelF& k) {
   return c;
 }
 
-bool pair_const_ok(const PairConst& c) {
+bool pair_const_ok(const ScannerF& s, const PairConst& c) {
   auto in = [](float v, float lo, float hi) { return v > lo && v < hi; };
-  return in(c.na4, 1e-25f, 1e25f) && in(c.na2, 1e-25f, 1e25f) && in(c.nb4, 1e-25f, 1e25f) &&
+  return s.min_closed_hw == 0.0f && in(c.na4, 1e-25f, 1e25f) && in(c.na2, 1e-25f, 1e25f) && in(c.nb4, 1e-25f, 1e25f) &&
          in(c.qm1, -0.999999f, 0.0f) && in(c.c9, 1e-25f, 1e25f);
 }
 
@@ -159,6 +159,12 @@ void dfree(T*& p) {
 int set_device(strip_ctx* ctx) {
   CK(cudaSetDevice(ctx->device));
   return STRIP_OK;
+}
+
+// Whether the row-pair kernels can take the context's geometry and sigmas.
+bool geometry_pairs(const strip_ctx* ctx) {
+  return pair_const_ok(
+      ctx->s, make_pair_const(ctx->s, make_kernel(ctx->g.sigma_z, ctx->g.sigma_dl, ctx->s.pw)));
 }
 
 // Chooses the tile size and halos for the largest event box, within the
@@ -207,14 +213,11 @@ Tiling choose_tiling(const strip_ctx* ctx, int max_w, int max_h) {
     if (HX >= HY) HX = HX * 3 / 4; else HY = HY * 3 / 4;
   }
   // column-major windows where they fit the same budget (fewer shared-memory
-  // bank conflicts in the walks); the row-pair kernels, which run there, need
-  // the closed form to settle every row and the kernel's constants in range
-  const bool pairs =
-      ctx->s.min_closed_hw == 0.0f &&
-      pair_const_ok(make_pair_const(
-          ctx->s, make_kernel(ctx->g.sigma_z, ctx->g.sigma_dl, ctx->s.pw)));
+  // bank conflicts in the walks), for every kernel; the tall ones for the
+  // row-pair kernels alone
+  const bool pairs = geometry_pairs(ctx);
   auto column_bytes = [&](int cs) { return 2 * t.WXmax * cs * 4; };
-  if (pairs && t.WYmax <= kColumnStride && column_bytes(kColumnStride) <= budget) {
+  if (t.WYmax <= kColumnStride && column_bytes(kColumnStride) <= budget) {
     t.cs = kColumnStride;
     t.smem_bytes = column_bytes(kColumnStride);
   } else if (pairs && max_h > kPairRows8 && max_h <= kPairRows16 &&
@@ -327,13 +330,14 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   std::vector<int64_t> gb(n_subsets), gc(n_subsets);
   const int64_t per_sub = (int64_t)(total / (unsigned long long)n_subsets) + 1;
   const int64_t target = (int64_t)ctx->sm_count * 2 * 8;
-  // Subsets of up to 1.2e6 events (column-major windows): a thousandth of the
+  // Subsets of up to 1.2e6 events (row-pair kernels): a thousandth of the
   // subset per item, between 128 and 1024, and no cut last wave -- two or three
   // waves of items that fill every warp.  Us per MLEM pass against 2048-event
   // items with the cut (one B200; 250 x 200 pixels of 2 mm / 800 x 400 of
   // 1 mm): 2e4 events 130 / 100 -> 55 / 64; 2e5 257 / 338 -> 235 / 285; 1e6
   // 827 / 1053 -> 820 / 990; 2e6 1539 / 1846 -> 1572 / 1827 (not taken).
-  const bool small = t.cs != 0 && ctx->tail_split && per_sub <= kSmallSubset;
+  const bool small =
+      t.cs != 0 && geometry_pairs(ctx) && ctx->tail_split && per_sub <= kSmallSubset;
   const int64_t chunk =
       ctx->item_events > 0
           ? std::min<int64_t>(kMaxItemEvents, ctx->item_events)
@@ -523,17 +527,21 @@ int check_ready(strip_ctx* ctx) {
   return STRIP_OK;
 }
 
-LaunchArgs base_args(strip_ctx* ctx) {
+// Arguments of a launch with the model's sigmas.  The GaussianKernel's launches
+// over column-major windows go to the row-pair kernels, which read the packs
+// (MLEM 3.47 against k_tile's 4.39 ms per 4e6 events, 800 x 400 pixels), where
+// these can take the constants.
+LaunchArgs base_args(strip_ctx* ctx, int mode, double sz, double sdl) {
   LaunchArgs a{};
   a.s = ctx->s;
-  a.k = make_kernel(ctx->g.sigma_z, ctx->g.sigma_dl, ctx->s.pw);
   a.t = ctx->t;
+  a.k = make_kernel(sz, sdl, ctx->s.pw);
+  a.pc = make_pair_const(a.s, a.k);
+  a.packs = mode == STRIP_MODE_CPU && pair_const_ok(a.s, a.pc) ? ctx->d_packs : nullptr;
   a.zu = ctx->d_zu;
   a.zd = ctx->d_zd;
   a.dl = ctx->d_dl;
   a.perm = ctx->d_perm;
-  a.packs = ctx->d_packs;
-  a.pc = make_pair_const(a.s, a.k);
   a.rho = ctx->d_rho;
   a.acc = ctx->d_acc;
   a.status = ctx->d_status;
@@ -543,6 +551,12 @@ LaunchArgs base_args(strip_ctx* ctx) {
   a.kbound = (float)((double)a.k.kc /
                      ((double)ctx->s.R * std::sqrt(2.0 * (double)a.k.ipsz)) * 1.02);
   a.n_fallback = ctx->d_fallback;
+  return a;
+}
+
+LaunchArgs mlem_args(strip_ctx* ctx, int mode) {
+  LaunchArgs a = base_args(ctx, mode, ctx->g.sigma_z, ctx->g.sigma_dl);
+  a.sens = (mode == STRIP_MODE_GPU) ? ctx->d_sens5 : nullptr;
   return a;
 }
 
@@ -831,8 +845,7 @@ int strip_iterate(strip_ctx* ctx, int n_iter, int mode, int n_subsets,
   if (int rc = ensure_binning(ctx, n_subsets)) return rc;
   if (mode == STRIP_MODE_GPU)
     if (int rc = ensure_sens5(ctx)) return rc;
-  LaunchArgs a = base_args(ctx);
-  a.sens = (mode == STRIP_MODE_GPU) ? ctx->d_sens5 : nullptr;
+  LaunchArgs a = mlem_args(ctx, mode);
   int launches = 0;
   // one event pair per tile launch, for the tile kernel's device time
   const size_t n_marks = (size_t)n_iter * ctx->n_subsets;
@@ -917,8 +930,7 @@ int strip_accumulate(strip_ctx* ctx, int mode, int n_subsets, int subset) {
   if (int rc = ensure_binning(ctx, n_subsets)) return rc;
   if (mode == STRIP_MODE_GPU)
     if (int rc = ensure_sens5(ctx)) return rc;
-  LaunchArgs a = base_args(ctx);
-  a.sens = (mode == STRIP_MODE_GPU) ? ctx->d_sens5 : nullptr;
+  LaunchArgs a = mlem_args(ctx, mode);
   set_subset(ctx, a, subset);
   CK(cudaMemsetAsync(ctx->d_fallback, 0, sizeof(unsigned long long), ctx->stream));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
@@ -961,9 +973,7 @@ int forward_dev(strip_ctx* ctx, const float* d_rho, double sz, double sdl,
   if (mode == STRIP_MODE_GPU)
     if (int rc = ensure_sens5(ctx)) return rc;
   CK(cudaMemsetAsync(d_y, 0, ctx->n_events * sizeof(double), ctx->stream));
-  LaunchArgs a = base_args(ctx);
-  a.k = make_kernel(sz, sdl, ctx->s.pw);
-  a.pc = make_pair_const(a.s, a.k);
+  LaunchArgs a = base_args(ctx, mode, sz, sdl);
   a.rho = d_rho;
   a.sens = (mode == STRIP_MODE_GPU) ? ctx->d_sens5 : nullptr;
   a.y_out = d_y;
@@ -980,15 +990,9 @@ int adjoint_dev(strip_ctx* ctx, const double* d_w, double sz, double sdl,
     CK(ev_alloc(ctx, &ctx->d_wbin, ctx->n_binned * sizeof(float)));
   CK(launch_gather_weights(ctx->d_perm, d_w, ctx->n_binned, ctx->d_wbin,
                            ctx->stream));
-  LaunchArgs a = base_args(ctx);
-  a.k = make_kernel(sz, sdl, ctx->s.pw);
-  a.pc = make_pair_const(a.s, a.k);
+  LaunchArgs a = base_args(ctx, mode, sz, sdl);
   a.acc = d_g;
   a.wf_in = ctx->d_wbin;
-  // GaussianKernel values are at most kc / sqrt(2 R^2 ipsz): E <= 1 and
-  // a'Sa >= ipsz (ap^2 + aq^2) >= 2 R^2 ipsz sec^4
-  a.kbound = (float)((double)a.k.kc /
-                     ((double)ctx->s.R * std::sqrt(2.0 * (double)a.k.ipsz)) * 1.02);
   if (int rc = run_all(ctx, OP_ADJOINT, mode, a)) return rc;
   if (mode == STRIP_MODE_GPU)
     CK(launch_scale_copy(d_g, ctx->d_sens5, d_g, ctx->n_pix, ctx->stream));
@@ -998,9 +1002,7 @@ int adjoint_dev(strip_ctx* ctx, const double* d_w, double sz, double sdl,
 int grad_dev(strip_ctx* ctx, const float* d_rho, const double* d_w, double sz,
              double sdl, double* d_out2) {
   CK(cudaMemsetAsync(d_out2, 0, 2 * sizeof(double), ctx->stream));
-  LaunchArgs a = base_args(ctx);
-  a.k = make_kernel(sz, sdl, ctx->s.pw);
-  a.pc = make_pair_const(a.s, a.k);
+  LaunchArgs a = base_args(ctx, STRIP_MODE_CPU, sz, sdl);
   a.rho = d_rho;
   a.w_in = d_w;
   a.grad_out = d_out2;
@@ -1265,8 +1267,7 @@ int ctx_prepare_mlem(strip_ctx* ctx, int mode) {
 }
 
 LaunchArgs ctx_mlem_args(strip_ctx* ctx, int mode) {
-  LaunchArgs a = base_args(ctx);
-  a.sens = (mode == STRIP_MODE_GPU) ? ctx->d_sens5 : nullptr;
+  LaunchArgs a = mlem_args(ctx, mode);
   if (ctx->sub_item_count.empty()) {
     a.items = ctx->d_items;
     a.n_items = 0;

@@ -120,8 +120,9 @@ struct PairConst {
   float cd, c1;         // log2 E = c1 t^2 + cd sec^2 dy^2
   float r1, r0, qm1;    // ratio 2^(r1 t + r0), ratio of ratios less one
 };
-// Whether the row-pair kernels can take the kernel's constants.
-bool pair_const_ok(const PairConst& c);
+// Whether the row-pair kernels can take the geometry (the closed form settles
+// every row) and the kernel's constants.
+bool pair_const_ok(const ScannerF& s, const PairConst& c);
 PairConst make_pair_const(const ScannerF& s, const KernelF& k);
 
 struct LaunchArgs {
@@ -131,7 +132,7 @@ struct LaunchArgs {
   const float* zu;    // events, binned order
   const float* zd;
   const float* dl;
-  const EventPack* packs;  // the same, set up (column-major windows)
+  const EventPack* packs;  // the same, set up: the launch is the row-pair kernels' (or null)
   PairConst pc;
   const int64_t* perm;   // binned position -> caller's event index
   const float* rho;      // image
@@ -189,6 +190,15 @@ struct BatchUpdateArgs {
 ScannerF make_scanner(const strip_geometry& g);
 KernelF make_kernel(double sigma_z, double sigma_dl, float pw);
 
+// Which windows a launch's kernels read: row-major (k_tile), column-major of
+// stride kColumnStride (k_tile or the row-pair kernels) or of kTallStride (the
+// row-pair kernels).
+enum Windows { kRowMajor, kColumns, kPairColumns, kPairTall };
+inline int windows_of(const LaunchArgs& a) {
+  if (a.packs) return a.t.cs == kTallStride ? kPairTall : kPairColumns;
+  return a.t.cs == kColumnStride ? kColumns : kRowMajor;
+}
+
 // ---- launchers (strip_kernels.cu) ----------------------------------------
 int tile_smem_bytes(int WYmax, int WS);
 cudaError_t launch_event_boxes(const ScannerF& s, const float* zu,
@@ -216,9 +226,9 @@ cudaError_t launch_item_order(const ScannerF& s, const Tiling& t, const WorkItem
                               int64_t* operm, EventPack* packs, cudaStream_t st);
 // GaussianKernel over column-major windows (strip_pairs.cu).
 cudaError_t launch_pair_tile(int op, int accum, const LaunchArgs& a, cudaStream_t st);
-cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int cs);
+cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int windows);
 cudaError_t launch_pair_batch(int accum, const BatchArgs& b, const BatchItem* items, int n_items,
-                              int* counter, int smem_bytes, int max_rows, int cs, int sm_count,
+                              int* counter, int smem_bytes, int max_rows, int windows, int sm_count,
                               cudaStream_t st);
 cudaError_t launch_global(int op, int mode, int accum, const LaunchArgs& a,
                           cudaStream_t st);
@@ -240,10 +250,11 @@ cudaError_t launch_gather_weights(const int64_t* perm, const double* w,
 // launch is captured into a graph).
 // max_rows: the most box rows of any event of the launch's members; cs:
 // their windows' column stride (0: row-major).
-cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max_rows, int cs);
+cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max_rows,
+                                    int windows);
 cudaError_t launch_tile_batch(int mode, int accum, const BatchArgs& b,
                               const BatchItem* items, int n_items, int* counter,
-                              int smem_bytes, int max_rows, int cs, int sm_count,
+                              int smem_bytes, int max_rows, int windows, int sm_count,
                               cudaStream_t st);
 cudaError_t launch_update_batch(const BatchUpdateArgs& u, int64_t max_pix,
                                 cudaStream_t st);

@@ -2,9 +2,9 @@
 //
 //   k_event_boxes / k_bin_keys / k_bin_scatter   one-time binning of the events
 //       into image tiles (events are iteration-invariant, so this is paid once)
-//   k_tile      the tile kernel (row-major windows and the
-//       AnalyticKernel; the GaussianKernel over column-major windows, the
-//       common case, is strip_pairs.cu's): one CTA per (tile, event chunk) work item.  The
+//   k_tile      the tile kernel (row-major windows, the AnalyticKernel, and
+//       model sigmas that the row-pair kernels cannot take; the GaussianKernel
+//       over column-major windows, the common case, is strip_pairs.cu's): one CTA per (tile, event chunk) work item.  The
 //       tile's window of the image (tile + halo) is staged in shared memory
 //       next to a shared-memory backprojection accumulator.  A warp takes one
 //       event at a time:
@@ -1457,11 +1457,6 @@ int grid_for(int64_t n, int per_block = kThreads, int cap = 148 * 16) {
 
 constexpr int kSetsCap = 64;
 
-// Column-major windows reach this file's kernels for the AnalyticKernel only
-// (the GaussianKernel: launch_pair_tile).
-template <int OP, int MODE>
-constexpr bool column_major() { return MODE != STRIP_MODE_CPU; }
-
 template <int OP, int MODE, int ACC, int LPE, int CS>
 cudaError_t launch_tile_cs(const LaunchArgs& a, cudaStream_t st) {
   const int smem = a.t.smem_bytes / 2 * tile_windows<OP>();
@@ -1477,9 +1472,7 @@ cudaError_t launch_tile_cs(const LaunchArgs& a, cudaStream_t st) {
 
 template <int OP, int MODE, int ACC, int LPE>
 cudaError_t launch_tile_lpe(const LaunchArgs& a, cudaStream_t st) {
-  if constexpr (column_major<OP, MODE>()) {
-    if (a.t.cs == kColumnStride) return launch_tile_cs<OP, MODE, ACC, LPE, kColumnStride>(a, st);
-  }
+  if (a.t.cs == kColumnStride) return launch_tile_cs<OP, MODE, ACC, LPE, kColumnStride>(a, st);
   return launch_tile_cs<OP, MODE, ACC, LPE, 0>(a, st);
 }
 
@@ -1523,8 +1516,7 @@ int tile_smem_bytes(int WYmax, int WS) { return 2 * WYmax * WS * 4; }
 cudaError_t launch_tile(int op, int mode, int accum, const LaunchArgs& a,
                         cudaStream_t st) {
   if (a.n_items <= 0) return cudaSuccess;
-  if (mode == STRIP_MODE_CPU && a.t.cs != 0)
-    return launch_pair_tile(op, accum, a, st);
+  if (a.packs) return launch_pair_tile(op, accum, a, st);
   switch (op) {
     case OP_MLEM:
       STRIP_DISPATCH(launch_tile_t, OP_MLEM, mode, accum, a, st);
@@ -1560,7 +1552,6 @@ cudaError_t launch_global(int op, int mode, int accum, const LaunchArgs& a,
 
 template <int THREADS, int CS, class F>
 cudaError_t with_tile_batch_t(int mode, int accum, bool half, F&& pick) {
-  if constexpr (CS == 0)  // column-major members of this mode: launch_pair_batch
   if (mode == STRIP_MODE_CPU) {
     constexpr int H = lanes_per_event<OP_MLEM, STRIP_MODE_CPU>();
     if (half) {
@@ -1586,23 +1577,24 @@ cudaError_t with_tile_batch_t(int mode, int accum, bool half, F&& pick) {
 // The persistent batch kernel of a class: windows that fit two CTAs per SM
 // run 512-thread CTAs, wider ones 1024-thread CTAs, one per SM; half-warp
 // events where every member's tallest box allows them; row-major or
-// column-major windows (cs).
+// column-major windows.
 template <class F>
-cudaError_t with_tile_batch(int mode, int accum, int smem_bytes, int max_rows, int cs,
+cudaError_t with_tile_batch(int mode, int accum, int smem_bytes, int max_rows, int windows,
                             F&& pick) {
   const bool half = half_warp_events(OP_MLEM, max_rows, true);
   const bool wide = smem_bytes > kNarrowSmemBytes;
-  if (cs == kColumnStride)
+  if (windows == kColumns)
     return wide ? with_tile_batch_t<kWideThreads, kColumnStride>(mode, accum, half, pick)
                 : with_tile_batch_t<kTileThreads, kColumnStride>(mode, accum, half, pick);
   return wide ? with_tile_batch_t<kWideThreads, 0>(mode, accum, half, pick)
               : with_tile_batch_t<kTileThreads, 0>(mode, accum, half, pick);
 }
 
-cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max_rows, int cs) {
-  if (mode == STRIP_MODE_CPU && cs != 0)
-    return pair_batch_reserve_smem(accum, smem_bytes, max_rows, cs);
-  return with_tile_batch(mode, accum, smem_bytes, max_rows, cs, [&](auto fn) {
+cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max_rows,
+                                    int windows) {
+  if (windows >= kPairColumns)
+    return pair_batch_reserve_smem(accum, smem_bytes, max_rows, windows);
+  return with_tile_batch(mode, accum, smem_bytes, max_rows, windows, [&](auto fn) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 smem_bytes);
   });
@@ -1610,19 +1602,19 @@ cudaError_t tile_batch_reserve_smem(int mode, int accum, int smem_bytes, int max
 
 cudaError_t launch_tile_batch(int mode, int accum, const BatchArgs& b,
                               const BatchItem* items, int n_items, int* counter,
-                              int smem_bytes, int max_rows, int cs, int sm_count,
+                              int smem_bytes, int max_rows, int windows, int sm_count,
                               cudaStream_t st) {
   if (n_items <= 0) return cudaSuccess;
-  if (mode == STRIP_MODE_CPU && cs != 0)
-    return launch_pair_batch(accum, b, items, n_items, counter, smem_bytes, max_rows, cs, sm_count,
-                             st);
+  if (windows >= kPairColumns)
+    return launch_pair_batch(accum, b, items, n_items, counter, smem_bytes, max_rows, windows,
+                             sm_count, st);
   const bool wide = smem_bytes > kNarrowSmemBytes;
   auto pick = [&](auto fn) -> cudaError_t {
     const int grid = std::min(n_items, sm_count * (wide ? 1 : 2));
     fn<<<grid, wide ? kWideThreads : kTileThreads, smem_bytes, st>>>(b, items, n_items, counter);
     return cudaGetLastError();
   };
-  return with_tile_batch(mode, accum, smem_bytes, max_rows, cs, pick);
+  return with_tile_batch(mode, accum, smem_bytes, max_rows, windows, pick);
 }
 
 

@@ -733,8 +733,8 @@ cudaError_t with_pair_batch_w(int accum, int smem_bytes, F&& pick) {
 }
 
 template <class F>
-cudaError_t with_pair_batch(int accum, int smem_bytes, int max_rows, int cs, F&& pick) {
-  if (cs == kTallStride)
+cudaError_t with_pair_batch(int accum, int smem_bytes, int max_rows, int windows, F&& pick) {
+  if (windows == kPairTall)
     return with_pair_batch_w<16, kBlocks16, kTallStride>(accum, smem_bytes, pick);
   if (max_rows > kPairRows8)
     return with_pair_batch_w<16, kBlocks16, kColumnStride>(accum, smem_bytes, pick);
@@ -743,17 +743,17 @@ cudaError_t with_pair_batch(int accum, int smem_bytes, int max_rows, int cs, F&&
 
 }  // namespace
 
-cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int cs) {
-  return with_pair_batch(accum, smem_bytes, max_rows, cs, [&](auto fn) {
+cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int windows) {
+  return with_pair_batch(accum, smem_bytes, max_rows, windows, [&](auto fn) {
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   });
 }
 
 cudaError_t launch_pair_batch(int accum, const BatchArgs& b, const BatchItem* items, int n_items,
-                              int* counter, int smem_bytes, int max_rows, int cs, int sm_count,
-                              cudaStream_t st) {
+                              int* counter, int smem_bytes, int max_rows, int windows,
+                              int sm_count,                               cudaStream_t st) {
   const bool wide = smem_bytes > kNarrowSmemBytes;
-  return with_pair_batch(accum, smem_bytes, max_rows, cs, [&](auto fn) -> cudaError_t {
+  return with_pair_batch(accum, smem_bytes, max_rows, windows, [&](auto fn) -> cudaError_t {
     const int grid = std::min(n_items, sm_count * (wide ? 1 : 2));
     fn<<<grid, wide ? kPairWide : kPairThreads, smem_bytes, st>>>(b, items, n_items, counter);
     return cudaGetLastError();

@@ -24,8 +24,9 @@
 // Accuracy.  q (the ratio of neighbouring ratios) would enter pixel j of a run
 // with its rounding error times j (j - 1) / 2.  The ratios advance by
 // R <- R + R (q - 1), one fused operation with q - 1 rounded: the error is
-// smaller by |q - 1| (0.08 at sigma_z = 5 pixels).  (Not in the sigma
-// gradient, which keeps the one-row kernel's steps.)
+// smaller by |q - 1| (0.08 at sigma_z = 5 pixels).  Below q = 1/2 it is larger,
+// and steep sigmas go to k_tile (pair_const_ok).  (Not in the sigma gradient,
+// which keeps the one-row kernel's steps.)
 //
 // Backprojection window: unsigned 32-bit fixed point as in strip_kernels.cu
 // (fixed_shift and the unweighted windows of strip_internal.h).  An addend

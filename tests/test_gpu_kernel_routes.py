@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as orc
-from test_gpu_row_pairs import CASES, IMAGE_TOL, events, rel
+from test_gpu_row_pairs import CASES, EVENT_TOL, IMAGE_TOL, events, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,29 @@ def test_batch_of_every_kind_of_window():
     finally:
         for rec in recs:
             rec.close()
+
+
+@pytest.mark.parametrize("sigma", [0.5, 0.6, 1.0, 2.0])
+def test_model_sigma_of_a_pixel_and_less(sigma):
+    """Projections with a model sigma_z below the geometry's 2 pixels.  All
+    coordinates are exact in binary32, so an event's error is that of the
+    run's first value, 2^-x at 2.12 geometry sigmas, and of the up to five
+    ratios to the row's largest pixel, each 2^r: two roundings of the exponent
+    each."""
+    import stripmlem as sm
+    case = (200.0, 500.0, 128, 128, 1.0, 2.0, 20.0)
+    g, n = geometry(case), 4_000
+    r = np.random.default_rng(0)
+    z = (r.integers(-40 * 64, 40 * 64, n) / 64.0).astype(np.float32)
+    dl = (r.integers(-60 * 32, 60 * 32, n) / 32.0).astype(np.float32)
+    rho = r.lognormal(0.0, 0.5, (128, 128)).astype(np.float32)
+    w = r.uniform(0.5, 2.0, n)
+    log2e, t = 1.4427, 2.12 * 2.0
+    x, ratio = log2e * t * t / sigma ** 2, log2e * (2 * t + 1) / sigma ** 2
+    tol = EVENT_TOL + 0.6931 * 2.0 ** -23 * (x + min(5.0, t) * ratio / 2)
+    with sm.Reconstruction(scanner(case)) as rec:
+        rec.set_events(z, z, dl)
+        y = rec.forward(rho, sigma, 20.0)
+        o = orc.forward_f64(g, z, z, dl, rho, sigma, 20.0)
+        assert np.abs(y / o - 1).max() < tol
+        assert rel(rec.adjoint(w, sigma, 20.0), orc.adjoint_f64(g, z, z, dl, w, sigma, 20.0)) < tol

@@ -213,8 +213,9 @@ int strip_batch_create(strip_ctx* const* members, int n_members, int mode,
     b->args->member[m] = ctx_mlem_args(c, mode);
     const bool own_launch =
         b->args->member[m].n_items >= STRIP_BATCH_SPLIT_PER_SM * b->sm_count;
-    const int cls =
-        (c->t.smem_bytes > kNarrowSmem) + 2 * windows_of(b->args->member[m]);
+    const bool wide = c->t.smem_bytes > kNarrowSmem;
+    const int windows = windows_of(b->args->member[m]), cls = wide + 2 * windows;
+    if (windows < kPairColumns) b->args->member[m].grab = tile_grab(b->args->member[m], wide);
     b->cls_smem[cls] = std::max(b->cls_smem[cls], c->t.smem_bytes);
     b->cls_rows[cls] = std::max(b->cls_rows[cls], c->t.max_rows);
     b->n_events += c->n_events;

@@ -337,18 +337,19 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   std::vector<int64_t> gb(n_subsets), gc(n_subsets);
   const int64_t per_sub = (int64_t)(total / (unsigned long long)n_subsets) + 1;
   const int64_t target = (int64_t)ctx->sm_count * 2 * 8;
-  // Subsets of up to 1.2e6 events (row-pair kernels): a thousandth of the
+  // Subsets of up to 1.2e6 events (column-major windows): a thousandth of the
   // subset per item, between 128 and 1024, and no cut last wave -- two or three
-  // waves of items that fill every warp.  Us per MLEM pass against 2048-event
-  // items with the cut (one B200; 250 x 200 pixels of 2 mm / 800 x 400 of
-  // 1 mm): 2e4 events 130 / 100 -> 55 / 64; 2e5 257 / 338 -> 235 / 285; 1e6
-  // 827 / 1053 -> 820 / 990; 2e6 1539 / 1846 -> 1572 / 1827 (not taken).
-  const bool small =
-      t.cs != 0 && geometry_pairs(ctx) && ctx->tail_split && per_sub <= kSmallSubset;
+  // waves of items that fill every warp (tile_grab, pair_tile_item).  Us per
+  // MLEM pass against 2048-event items with the cut (one B200; 250 x 200 pixels
+  // of 2 mm / 800 x 400 of 1 mm), GaussianKernel: 2e4 events 130 / 100 -> 55 /
+  // 64; 2e5 257 / 338 -> 235 / 285; 1e6 827 / 1053 -> 820 / 990; 2e6 1539 / 1846
+  // -> 1572 / 1827 (not taken).  AnalyticKernel: 2e4 433 / 878 -> 174 / 194; 2e5
+  // 1054 / 1477 -> 845 / 932; 1e6 3702 / 4251 -> 3710 / 4100.
+  const bool small = t.cs != 0 && ctx->tail_split && per_sub <= kSmallSubset;
   const int64_t chunk =
       ctx->item_events > 0
           ? std::min<int64_t>(kMaxItemEvents, ctx->item_events)
-      : small ? std::min<int64_t>(1024, std::max<int64_t>(128, per_sub / 1000))
+      : small ? std::min<int64_t>(kSmallItem, std::max<int64_t>(128, per_sub / 1000))
               : std::min<int64_t>(kMaxItemEvents,
                                   std::max<int64_t>(2048, per_sub / target + 1));
   for (int sb = 0; sb < n_subsets; ++sb) {
@@ -553,6 +554,7 @@ LaunchArgs base_args(strip_ctx* ctx, int mode, double sz, double sdl) {
   a.acc = ctx->d_acc;
   a.status = ctx->d_status;
   a.grab = ctx->grab;
+  a.item_events = ctx->stats.max_item_events;
   // GaussianKernel values are at most kc / sqrt(2 R^2 ipsz): E <= 1 and
   // a'Sa >= ipsz (ap^2 + aq^2) >= 2 R^2 ipsz sec^4
   a.kbound = (float)((double)a.k.kc /

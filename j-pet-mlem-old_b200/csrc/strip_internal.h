@@ -74,6 +74,8 @@ constexpr int kColumnStride = 128, kTallStride = 160;
 // The most box rows of the row-pair kernels' lane layouts (8 and 16 lanes an
 // event).
 constexpr int kPairRows8 = 80, kPairRows16 = 128;
+// The largest of the small work items (events).
+constexpr int kSmallItem = 1024;
 
 __host__ __device__ inline void tile_window(const Tiling& t, int n_z, int n_y,
                                             int tile, int& wx0, int& wy0,
@@ -150,6 +152,7 @@ struct LaunchArgs {
   float kbound;          // bound of the GaussianKernel values (OP_ADJOINT,
                          // OP_MLEM with the reference CPU semantics)
   int grab;              // events a warp takes per counter step (1..32)
+  int item_events;       // of the largest work item
   int* status;           // device status word (0 = ok)
   // OP_MLEM, GaussianKernel: per work item (indexed like `items`), the
   // item's sum of 1 / D_e times its window's mean image value from the last
@@ -201,6 +204,8 @@ inline int windows_of(const LaunchArgs& a) {
 
 // ---- launchers (strip_kernels.cu) ----------------------------------------
 int tile_smem_bytes(int WYmax, int WS);
+// The events k_tile's warps take per counter step (at most a.grab).
+int tile_grab(const LaunchArgs& a, bool wide);
 cudaError_t launch_event_boxes(const ScannerF& s, const float* zu,
                                const float* zd, const float* dl, int64_t n,
                                int4* boxes, int* max_wh, unsigned long long* n_empty,

@@ -841,8 +841,7 @@ __device__ __forceinline__ void tile_item(const LaunchArgs& a,
   float wsum = 0.0f;
   // window word of (row r, column c): row-major or column-major (CS)
   auto widx = [WS](int r, int c) { return CS ? c * CS + r : r * WS + c; };
-  for (int q = threadIdx.x; q < wxn * wyn; q += blockDim.x) {
-    const int r = q / wxn, c = q - r * wxn;
+  each_pixel<CS != 0>(wxn, wyn, lane, [&](int r, int c) {
     const int64_t gi = (int64_t)(wy0 + r) * a.s.n_z + wx0 + c;
     if (kReads) {
       float v = a.rho[gi];
@@ -851,7 +850,7 @@ __device__ __forceinline__ void tile_item(const LaunchArgs& a,
       wsum += v;
     }
     if (kWrites) s_acc[widx(r, c)] = 0.0f;
-  }
+  });
   __syncthreads();
   const uint32_t w_sh = (uint32_t)__cvta_generic_to_shared(s_w);
   const uint32_t acc_sh = (uint32_t)__cvta_generic_to_shared(s_acc);
@@ -861,8 +860,7 @@ __device__ __forceinline__ void tile_item(const LaunchArgs& a,
   auto flush = [&](int fshift, bool unweighted) {
     unsigned* s_acc_u = reinterpret_cast<unsigned*>(s_acc);
     const int* s_acc_i = reinterpret_cast<const int*>(s_acc);
-    for (int q = threadIdx.x; q < wxn * wyn; q += blockDim.x) {
-      const int r = q / wxn, c = q - r * wxn;
+    each_pixel<CS != 0>(wxn, wyn, lane, [&](int r, int c) {
       double v;
       const int wi = widx(r, c);
       if constexpr (kFixedMlem) {
@@ -878,7 +876,7 @@ __device__ __forceinline__ void tile_item(const LaunchArgs& a,
       }
       if (v != 0.0)
         atomicAdd(a.acc + (int64_t)(wy0 + r) * a.s.n_z + wx0 + c, v);
-    }
+    });
   };
   // A weighted MLEM window over `count` events of the item (those of `only`,
   // or all); returns its scale's exponent.
@@ -1458,7 +1456,7 @@ int grid_for(int64_t n, int per_block = kThreads, int cap = 148 * 16) {
 constexpr int kSetsCap = 64;
 
 template <int OP, int MODE, int ACC, int LPE, int CS>
-cudaError_t launch_tile_cs(const LaunchArgs& a, cudaStream_t st) {
+cudaError_t launch_tile_cs(LaunchArgs a, cudaStream_t st) {
   const int smem = a.t.smem_bytes / 2 * tile_windows<OP>();
   const bool wide = smem > kNarrowSmemBytes;  // one CTA per SM: 1024 threads
   auto fn = wide ? k_tile<OP, MODE, ACC, kWideThreads, LPE, CS>
@@ -1466,6 +1464,7 @@ cudaError_t launch_tile_cs(const LaunchArgs& a, cudaStream_t st) {
   cudaError_t err = cudaFuncSetAttribute(
       fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) return err;
+  a.grab = tile_grab(a, wide);
   fn<<<a.n_items, wide ? kWideThreads : kTileThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
@@ -1509,6 +1508,18 @@ cudaError_t launch_global_t(const LaunchArgs& a, cudaStream_t st) {
       return FN<op, STRIP_MODE_GPU, STRIP_ACCUM_FP64>(a, st);              \
     return FN<op, STRIP_MODE_GPU, STRIP_ACCUM_KAHAN>(a, st);               \
   } while (0)
+
+// Small work items (tilings with column-major windows have them): as many
+// counter steps as give every warp the same number.  Set on the host: in the
+// kernel it costs registers (2-5 % of a pass).  AnalyticKernel, us per MLEM pass
+// (200 x 250 pixels of 2 mm; steps of 32 -> these): 2e4 events 429 -> 174, 1e5
+// 1150 -> 455, 2e5 1587 -> 845, 5e5 1978 -> 1973.
+int tile_grab(const LaunchArgs& a, bool wide) {
+  if (a.t.cs == 0 || a.item_events > kSmallItem || a.item_events <= 0) return a.grab;
+  const int warps = (wide ? kWideThreads : kTileThreads) / 32;
+  const int steps = (a.item_events - 1) / (a.grab * warps) + 1;
+  return (a.item_events - 1) / (steps * warps) + 1;
+}
 
 // Two windows (the image and the accumulator) of WYmax rows of stride WS.
 int tile_smem_bytes(int WYmax, int WS) { return 2 * WYmax * WS * 4; }

@@ -511,17 +511,7 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
     for (int q = threadIdx.x; q < kMaxItemEvents / 32; q += blockDim.x) s_fb_bits[q] = 0u;
   const int lane = threadIdx.x & 31;
   float wsum = 0.0f;
-  // f(row, column) over the window, a warp taking 8 rows x 4 columns at a time:
-  // 4-way shared-memory conflicts (a row of 32 columns: 32-way) and whole
-  // sectors of the image in L1
-  auto each = [&](auto f) {
-    const int n_ct = (wxn + 3) >> 2, n_t = n_ct * ((wyn + 7) >> 3);
-    for (int t = threadIdx.x >> 5; t < n_t; t += blockDim.x >> 5) {
-      const int rt = t / n_ct, r = 8 * rt + (lane & 7), c = 4 * (t - rt * n_ct) + (lane >> 3);
-      if (r < wyn && c < wxn) f(r, c);
-    }
-  };
-  each([&](int r, int c) {
+  each_pixel<true>(wxn, wyn, lane, [&](int r, int c) {
     if (kReads) {
       const float v = a.rho[(int64_t)(wy0 + r) * a.s.n_z + wx0 + c];
       s_w[c * CS + r] = v;
@@ -542,7 +532,7 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
   // the global binary64 accumulator.
   auto flush = [&](int fshift, bool unweighted) {
     const double per = exp2((double)-fshift);
-    each([&](int r, int c) {
+    each_pixel<true>(wxn, wyn, lane, [&](int r, int c) {
       const int wi = c * CS + r;
       const unsigned raw = __float_as_uint(s_acc[wi]);
       double v = (OP == OP_ADJOINT ? (double)(int)raw : (double)raw) * per;

@@ -107,6 +107,26 @@ __device__ int adjoint_shift(const LaunchArgs& a, const WorkItem& it, int lane,
   return s_shift;
 }
 
+// f(row, column) over a window of wyn rows and wxn columns.  Column-major, a warp
+// takes 8 rows x 4 columns at a time: 4-way shared-memory conflicts (a row of
+// 32 columns: 32-way) and whole sectors of the image in L1; row-major, the rows
+// one after the other.
+template <bool COLUMNS, class F>
+__device__ __forceinline__ void each_pixel(int wxn, int wyn, int lane, F&& f) {
+  if constexpr (COLUMNS) {
+    const int n_ct = (wxn + 3) >> 2, n_t = n_ct * ((wyn + 7) >> 3);
+    for (int t = threadIdx.x >> 5; t < n_t; t += blockDim.x >> 5) {
+      const int rt = t / n_ct, r = 8 * rt + (lane & 7), c = 4 * (t - rt * n_ct) + (lane >> 3);
+      if (r < wyn && c < wxn) f(r, c);
+    }
+  } else {
+    for (int q = threadIdx.x; q < wxn * wyn; q += blockDim.x) {
+      const int r = q / wxn;
+      f(r, q - r * wxn);
+    }
+  }
+}
+
 // Sum of v over the CTA, returned to every thread (two barriers).
 __device__ __forceinline__ float block_sum(float v) {
   __shared__ float s_part[kMaxWarps];

@@ -435,6 +435,18 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
     if (e == cudaSuccess)
       e = launch_item_order(ctx->s, t, d_items, (int)items.size(), ozu, ozd, odl, operm, qzu,
                             qzd, qdl, qperm, packs, st);
+    // the events of the global path, in no item, keep their places
+    for (int sb = 0; sb < n_subsets; ++sb) {
+      auto keep = [&](auto* to, const auto* from) {
+        if (e == cudaSuccess && gc[sb] > 0)
+          e = cudaMemcpyAsync(to + gb[sb], from + gb[sb], gc[sb] * sizeof(*to),
+                              cudaMemcpyDeviceToDevice, st);
+      };
+      keep(qzu, ozu);
+      keep(qzd, ozd);
+      keep(qdl, odl);
+      keep(qperm, operm);
+    }
     if (e != cudaSuccess) {
       ev_free(ctx, qzu);
       ev_free(ctx, qzd);

@@ -91,3 +91,32 @@ def test_model_sigma_of_a_pixel_and_less(sigma):
         o = orc.forward_f64(g, z, z, dl, rho, sigma, 20.0)
         assert np.abs(y / o - 1).max() < tol
         assert rel(rec.adjoint(w, sigma, 20.0), orc.adjoint_f64(g, z, z, dl, w, sigma, 20.0)) < tol
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_overflow_events_of_column_major_tilings(mode):
+    """Boxes too wide for any tile's halo beside an image of few rows: those
+    events take the global path, the others column-major windows."""
+    import stripmlem as sm
+    case = (300.0, 900.0, 120, 400, 1.0, 20.0, 110.0)
+    g, s_z, s_dl = geometry(case), case[5], case[6]
+    r = np.random.default_rng(3)
+    n = 900
+    z, y = r.uniform(-190.0, 190.0, n), r.uniform(-58.0, 58.0, n)
+    t = np.where(np.arange(n) % 3 == 0, r.uniform(0.9, 1.2, n), r.uniform(-0.2, 0.2, n))
+    ev = [v.astype(np.float32) for v in (z + (300.0 - y) * t, z - (300.0 + y) * t,
+                                         -2 * y * np.sqrt(1 + t * t))]
+    rho = r.lognormal(0.0, 0.5, (120, 400)).astype(np.float32)
+    w = r.uniform(0.5, 2.0, n)
+    with sm.Reconstruction(scanner(case), mode=mode) as rec:
+        for n_subsets in (1, 3):
+            rec.set_events(*ev, n_subsets=n_subsets)
+            st = rec.stats()
+            assert 0 < st["n_overflow"] < n and st["smem_bytes"] % 1024 == 0
+            y = rec.forward(rho, s_z, s_dl)
+            assert rel(y, orc.forward_f64(g, *ev, rho, s_z, s_dl, mode=mode)) < IMAGE_TOL
+            a = rec.adjoint(w, s_z, s_dl)
+            assert rel(a, orc.adjoint_f64(g, *ev, w, s_z, s_dl, mode=mode)) < IMAGE_TOL
+            rec.rho = np.ones((120, 400), np.float32)
+            rec(None, 2)
+            assert rel(rec.rho, orc.mlem_f64(g, *ev, 2, mode=mode, n_subsets=n_subsets)) < IMAGE_TOL

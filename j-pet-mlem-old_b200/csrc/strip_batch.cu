@@ -60,6 +60,7 @@ struct strip_batch {
   int accum = STRIP_ACCUM_KAHAN;
   int sm_count = 148;
   std::vector<strip_ctx*> members;
+  std::vector<std::shared_ptr<char>> in_batch;  // the members' shares (strip_ctx.h)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   BatchArgs* args = nullptr;  // host copy of the kernel parameters (~20 KB)
@@ -211,6 +212,7 @@ int strip_batch_create(strip_ctx* const* members, int n_members, int mode,
       }
     }
     b->args->member[m] = ctx_mlem_args(c, mode);
+    b->in_batch.push_back(c->in_batch);
     const bool own_launch =
         b->args->member[m].n_items >= STRIP_BATCH_SPLIT_PER_SM * b->sm_count;
     const bool wide = c->t.smem_bytes > kNarrowSmem;

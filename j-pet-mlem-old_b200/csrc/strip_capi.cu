@@ -245,6 +245,21 @@ Tiling choose_tiling(const strip_ctx* ctx, int max_w, int max_h) {
   return t;
 }
 
+// The events set up for the row-pair kernels (24 bytes each), made by the first
+// launch that reads them, so that a context of the AnalyticKernel alone has
+// none; null without memory for them.
+const EventPack* event_packs(strip_ctx* ctx) {
+  if (!ctx->d_packs && ctx->n_binned > 0) {
+    if (ev_alloc(ctx, &ctx->d_packs, ctx->n_binned * sizeof(EventPack)) != cudaSuccess ||
+        launch_event_packs(ctx->s, ctx->d_zu, ctx->d_zd, ctx->d_dl, ctx->n_binned, ctx->d_packs,
+                           ctx->stream) != cudaSuccess) {
+      cudaGetLastError();
+      ev_free(ctx, ctx->d_packs);
+    }
+  }
+  return ctx->d_packs;
+}
+
 // Sorts events (device arrays; `orig` maps them to the caller's indices or is
 // null for identity) into (subset, tile) bins and builds the work items.
 // On success the context owns the new binned arrays.
@@ -260,7 +275,11 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   unsigned long long* d_hist = nullptr;
   float *ozu = nullptr, *ozd = nullptr, *odl = nullptr;
   int64_t* operm = nullptr;
+  // The old events' packs make room: a binning needs 72 bytes an event at its
+  // peak (96 in a batch, whose graph reads them until it is destroyed).
+  const bool had_packs = ctx->d_packs != nullptr;
   EventPack* packs = nullptr;
+  if (ctx->in_batch.use_count() == 1) ev_free(ctx, ctx->d_packs);
   auto cleanup = [&]() {
     ev_free(ctx, packs);
     ev_free(ctx, boxes);
@@ -431,7 +450,13 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
     if (e == cudaSuccess) e = ev_alloc(ctx, &qzd, nb * sizeof(float));
     if (e == cudaSuccess) e = ev_alloc(ctx, &qdl, nb * sizeof(float));
     if (e == cudaSuccess) e = ev_alloc(ctx, &qperm, nb * sizeof(int64_t));
-    if (e == cudaSuccess) e = ev_alloc(ctx, &packs, nb * sizeof(EventPack));
+    // a context that has used packs gets the new ones on the way, given memory (a
+    // launch of their own: 661 against 653 us from 2e4 events to the image)
+    if (e == cudaSuccess && had_packs &&
+        ev_alloc(ctx, &packs, nb * sizeof(EventPack)) != cudaSuccess) {
+      cudaGetLastError();
+      packs = nullptr;
+    }
     if (e == cudaSuccess)
       e = launch_item_order(ctx->s, t, d_items, (int)items.size(), ozu, ozd, odl, operm, qzu,
                             qzd, qdl, qperm, packs, st);
@@ -550,14 +575,15 @@ int check_ready(strip_ctx* ctx) {
 // Arguments of a launch with the model's sigmas.  The GaussianKernel's launches
 // over column-major windows go to the row-pair kernels, which read the packs
 // (MLEM 3.47 against k_tile's 4.39 ms per 4e6 events, 800 x 400 pixels), where
-// these can take the constants.
+// these can take the constants and the packs have room.
 LaunchArgs base_args(strip_ctx* ctx, int mode, double sz, double sdl) {
   LaunchArgs a{};
   a.s = ctx->s;
   a.t = ctx->t;
   a.k = make_kernel(sz, sdl, ctx->s.pw);
   a.pc = make_pair_const(a.s, a.k);
-  a.packs = mode == STRIP_MODE_CPU && pair_const_ok(a.s, a.pc) ? ctx->d_packs : nullptr;
+  a.packs = mode == STRIP_MODE_CPU && a.t.cs != 0 && pair_const_ok(a.s, a.pc)
+                ? event_packs(ctx) : nullptr;
   a.zu = ctx->d_zu;
   a.zd = ctx->d_zd;
   a.dl = ctx->d_dl;

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -42,7 +43,9 @@ struct strip_ctx {
   float* d_zd = nullptr;
   float* d_dl = nullptr;
   int64_t* d_perm = nullptr;
-  stripmlem::EventPack* d_packs = nullptr;  // set-up events (column-major windows)
+  stripmlem::EventPack* d_packs = nullptr;  // set-up events (event_packs), or none yet
+  // a share is held by each batch whose captured graph reads d_packs
+  std::shared_ptr<char> in_batch = std::make_shared<char>();
   int n_subsets = 0;
   stripmlem::Tiling t{};
   int max_w = 0, max_h = 0;

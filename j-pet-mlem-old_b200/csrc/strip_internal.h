@@ -224,12 +224,15 @@ cudaError_t launch_tile(int op, int mode, int accum, const LaunchArgs& a,
                         cudaStream_t st);
 // The events of each work item (binned arrays zu.. perm) reordered into
 // ozu.. operm for the column-major windows' banks (k_item_order), and set up
-// into packs.
+// into packs (or null).
 cudaError_t launch_item_order(const ScannerF& s, const Tiling& t, const WorkItem* items,
                               int n_items, const float* zu, const float* zd, const float* dl,
                               const int64_t* perm, float* ozu, float* ozd, float* odl,
                               int64_t* operm, EventPack* packs, cudaStream_t st);
-// GaussianKernel over column-major windows (strip_pairs.cu).
+// GaussianKernel over column-major windows (strip_pairs.cu); their events, set
+// up.
+cudaError_t launch_event_packs(const ScannerF& s, const float* zu, const float* zd,
+                               const float* dl, int64_t n, EventPack* packs, cudaStream_t st);
 cudaError_t launch_pair_tile(int op, int accum, const LaunchArgs& a, cudaStream_t st);
 cudaError_t pair_batch_reserve_smem(int accum, int smem_bytes, int max_rows, int windows);
 cudaError_t launch_pair_batch(int accum, const BatchArgs& b, const BatchItem* items, int n_items,

@@ -1300,7 +1300,7 @@ __global__ void k_item_order(ScannerF s, Tiling t, const WorkItem* __restrict__ 
     ozd[o] = zd[i];
     odl[o] = dl[i];
     operm[o] = perm[i];
-    packs[o] = pack_event(e);
+    if (packs) packs[o] = pack_event(e);
   }
 }
 

@@ -120,3 +120,48 @@ def test_overflow_events_of_column_major_tilings(mode):
             rec.rho = np.ones((120, 400), np.float32)
             rec(None, 2)
             assert rel(rec.rho, orc.mlem_f64(g, *ev, 2, mode=mode, n_subsets=n_subsets)) < IMAGE_TOL
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_memory_of_replaced_events(mode):
+    """Device memory a context holds once its events were replaced.  The peak of
+    a binning is 72 bytes an event; the row-pair kernels' packs (24) are made
+    after it, of memory that it gave back or of their own."""
+    import torch
+    import stripmlem as sm
+    case = CASES[0]
+    n = 12_000_000
+    r = np.random.default_rng(4)
+    z, t, dl = (r.uniform(-b, b, n).astype(np.float32) for b in (200.0, 0.3, 300.0))
+    zu, zd = z + 200 * t, z - 200 * t
+    with sm.Reconstruction(scanner(case), mode=mode) as rec:
+        rec.set_events(zu[:9_000], zd[:9_000], dl[:9_000])
+        rec(None, 2)  # the kernels are loaded
+        free = torch.cuda.mem_get_info()[0]
+        for _ in range(2):
+            rec.set_events(zu, zd, dl)
+            rec(None, 1)
+        held = free - torch.cuda.mem_get_info()[0]
+    assert held < (72 + 24 + 4) * n
+
+
+def test_events_replaced_and_subsets_changed_between_kernels():
+    """The packs follow the binning: passes of both kernels, projections and
+    re-binnings in turn equal fresh contexts'."""
+    import stripmlem as sm
+    case = CASES[0]
+    s_z, s_dl = case[5:]
+    rho = np.random.default_rng(8).lognormal(0.0, 0.5, (case[2], case[3])).astype(np.float32)
+    with sm.Reconstruction(scanner(case)) as rec:
+        for seed, n, n_subsets in ((1, 5_000, 1), (2, 9_000, 2), (3, 700, 1)):
+            ev = events(case, n, seed)
+            g = geometry(case)
+            rec.set_events(*ev)
+            rec.rho = np.ones_like(rho)
+            rec(None, 1, mode=sm.MODE_GPU)
+            assert rel(rec.rho, orc.mlem_f64(g, *ev, 1, mode=1)) < IMAGE_TOL
+            rec.rho = np.ones_like(rho)
+            rec(None, 2, n_subsets=n_subsets)
+            assert rel(rec.rho, orc.mlem_f64(g, *ev, 2, n_subsets=n_subsets)) < IMAGE_TOL
+            y = rec.forward(rho, s_z, s_dl)
+            assert rel(y, orc.forward_f64(g, *ev, rho, s_z, s_dl)) < IMAGE_TOL

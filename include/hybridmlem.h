@@ -222,6 +222,10 @@ int hybrid_smear_responses(int64_t seed, double sigma_z, double sigma_dl, int64_
 int hybrid_debug_atan2(int32_t device, const float* a, const float* b, int64_t n,
                        int32_t which, float* out);
 
+/* Test hook: how many of the resident frame events the windowed iteration
+ * takes, and its work items and tasks (0: the per-event kernel takes all). */
+int hybrid_debug_windows(hybrid_ctx* ctx, int64_t* events, int64_t* items, int64_t* tasks);
+
 /* A z-cylinder of a synthetic phantom: centre, radius, half length along z,
  * activity. */
 typedef struct hybrid_cylinder {

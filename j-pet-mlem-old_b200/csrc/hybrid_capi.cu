@@ -831,6 +831,14 @@ int hybrid_get_stats(hybrid_ctx* ctx, hybrid_stats* out) {
   return STRIP_OK;
 }
 
+int hybrid_debug_windows(hybrid_ctx* ctx, int64_t* events, int64_t* items, int64_t* tasks) {
+  if (!ctx) return STRIP_E_INVALID;
+  if (events) *events = ctx->win.n_events;
+  if (items) *items = ctx->win.n_items;
+  if (tasks) *tasks = ctx->win.n_tasks;
+  return STRIP_OK;
+}
+
 int hybrid_debug_atan2(int32_t device, const float* a, const float* b, int64_t n,
                        int32_t which, float* out) {
   if (n < 0 || (n > 0 && (!a || !b || !out)) || (which != 0 && which != 1))

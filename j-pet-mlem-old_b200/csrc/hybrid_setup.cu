@@ -7,6 +7,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <cuda/std/functional>
 
 #include "hybrid_internal.h"
 
@@ -189,8 +190,10 @@ void launch_compact(const Frame* frames, const int32_t* keep, const int64_t* off
 namespace {
 
 // Sort keys: (LOR, plane slab); the largest key for an event no window takes
-// (counted).
-__global__ void k_order_keys(const Frame* __restrict__ frames, int32_t n, int64_t n_lors,
+// (counted): one without voxels or with more than a window holds, or whose
+// infos are not its LOR's (and the one after them, where a frame may end), so
+// that an item spans one LOR's infos however far apart its events' lie.
+__global__ void k_order_keys(const Frame* __restrict__ frames, int32_t n, const GeometryDev geo,
                              const WinPlan w, uint64_t* keys, int32_t* index,
                              int32_t* n_general) {
   for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -198,10 +201,11 @@ __global__ void k_order_keys(const Frame* __restrict__ frames, int32_t n, int64_
     uint64_t key = (uint64_t)f.lor;
     if (w.planes > 0) {
       const int rows = f.info_end - f.info_begin, planes = f.plane_end - f.plane_begin;
-      if (rows > 0 && planes > 0 && rows < (1 << kWinRowBits) && planes <= w.max_planes) {
+      if (rows > 0 && planes > 0 && rows < (1 << kWinRowBits) && planes <= w.max_planes &&
+          f.info_begin >= geo.lbeg[f.lor] && f.info_end <= geo.lend[f.lor] + 1) {
         key = key * w.n_slabs + f.plane_begin / w.tile_planes;
       } else {
-        key = (uint64_t)n_lors * w.n_slabs;
+        key = (uint64_t)geo.n_lors * w.n_slabs;
         atomicAdd(n_general, 1);
       }
     }
@@ -299,6 +303,14 @@ __global__ void k_item_tasks(const Frame* __restrict__ frames, const WinItem* __
   if (lane == 0 && sum) atomicAdd(entries, sum);
 }
 
+// Exclusive sums of 32-bit counts in 64 bits (DeviceScan adds in its initial
+// value's type; ExclusiveSum's is the input's).
+cudaError_t scan64(void* temp, size_t* temp_bytes, const int32_t* v, int64_t* out, int32_t n,
+                   cudaStream_t st) {
+  return cub::DeviceScan::ExclusiveScan(temp, *temp_bytes, v, out, cuda::std::plus<>{},
+                                        int64_t{0}, n, st);
+}
+
 }  // namespace
 
 cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* frames, int32_t n,
@@ -321,7 +333,7 @@ cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* fr
   cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, kn, kn, in, in, n, 0,
                                                   end_bit, st);
   if (e == cudaSuccess)
-    e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, in, on, n, st);
+    e = scan64(nullptr, &scan_bytes, in, on, n, st);
   if (e != cudaSuccess) return e;
   const size_t temp_bytes = std::max(sort_bytes, scan_bytes);
   void* block = nullptr;
@@ -354,7 +366,7 @@ cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* fr
   // total of an exclusive scan: its last offset plus the last value
   auto scan_total = [&](const int32_t* v, int32_t count, int64_t* total) {
     size_t tb = temp_bytes;
-    cudaError_t r = cub::DeviceScan::ExclusiveSum(temp, tb, v, offs, count, st);
+    cudaError_t r = scan64(temp, &tb, v, offs, count, st);
     int64_t last = 0;
     int32_t last_v = 0;
     if (r == cudaSuccess)
@@ -366,7 +378,7 @@ cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* fr
     return r;
   };
   STEP(cudaMemsetAsync(totals, 0, 16, st));
-  k_order_keys<<<grid_for(n), 256, 0, st>>>(frames, n, geo.n_lors, plan, keys, index, d_general);
+  k_order_keys<<<grid_for(n), 256, 0, st>>>(frames, n, geo, plan, keys, index, d_general);
   size_t tb = temp_bytes;
   STEP(cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys_out, index, index_out, n, 0, end_bit,
                                        st));

@@ -285,6 +285,7 @@ SIGNATURES.update({
     "hybrid_update": (ctypes.c_int, [_ctx]),
     "hybrid_get_image": (ctypes.c_int, [_ctx, _vp]),
     "hybrid_get_stats": (ctypes.c_int, [_ctx, _P(HybridStats)]),
+    "hybrid_debug_windows": (ctypes.c_int, [_ctx] + [_P(ctypes.c_int64)] * 3),
     "hybrid_debug_atan2": (ctypes.c_int, [ctypes.c_int32, _vp, _vp, ctypes.c_int64,
                                           ctypes.c_int32, _vp]),
     "hybrid_smear_responses": (ctypes.c_int, [ctypes.c_int64, ctypes.c_double, ctypes.c_double,

@@ -511,15 +511,19 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
     for (int q = threadIdx.x; q < kMaxItemEvents / 32; q += blockDim.x) s_fb_bits[q] = 0u;
   const int lane = threadIdx.x & 31;
   float wsum = 0.0f;
+  bool odd = false;  // a pixel below zero, infinite or NaN
   each_pixel<true>(wxn, wyn, lane, [&](int r, int c) {
     if (kReads) {
       const float v = a.rho[(int64_t)(wy0 + r) * a.s.n_z + wx0 + c];
       s_w[c * CS + r] = v;
-      wsum += v;
+      if (OP == OP_MLEM) {
+        wsum += v;
+        odd |= !(v >= 0.0f && v <= 3.402823466e38f);
+      }
     }
     if (kWrites) s_acc[c * CS + r] = 0.0f;
   });
-  __syncthreads();
+  odd = __syncthreads_or(odd);
   PairWin win{(uint32_t)__cvta_generic_to_shared(s_w), (uint32_t)__cvta_generic_to_shared(s_acc),
               wx0, wy0, 1.0f};
   // groups of events per counter step: fewer for small items, so that every
@@ -622,8 +626,9 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
     if (n_weighted > 0) {
       const int fs = fixed_shift(n_weighted);
       win.unit = exp2f((float)fs);
-      // K rho / D <= 1: addends up to the unit
-      if (fs <= 23)
+      // K rho / D <= 1: addends up to the unit; over images that updates made
+      // infinite, say, they may be anything, which cvt.rni clamps
+      if (fs <= 23 && !odd)
         pair_item<OP, ACC, LPE, NB, CS, true, kAddWeightedSubnormal>(a, it, win, lane, grab,
                                                                  s_next_group, only);
       else

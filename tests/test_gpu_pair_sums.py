@@ -1,0 +1,38 @@
+"""What the row-pair kernels add up, where a sum's form shows."""
+import numpy as np
+import pytest
+
+import stripmlem as sm
+from oracle import oracle as orc
+from test_gpu_row_pairs import CASES, IMAGE_TOL, events, rel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("accum", [sm.ACCUM_FP32, sm.ACCUM_KAHAN, sm.ACCUM_FP64])
+def test_pixels_that_an_update_made_infinite(accum):
+    """Events that see an infinite pixel have an infinite denominator and add
+    nothing, to that pixel either; the others are what they are without it."""
+    R, L, n_y, n_z, p, s_z, s_dl = case = CASES[5]
+    g, ev = orc.geometry(R, L, n_y, n_z, p, p, s_z, s_dl), events(CASES[5], 6_001, 6)
+    with sm.Reconstruction(sm.Scanner(R, L, n_y, n_z, p, p, s_z, s_dl),
+                           accumulation=accum) as rec:
+        rec.set_item_events(8000)  # one item: the conversion by subnormal products
+        rec.set_events(*ev)
+        rec(None, 2)
+        scale = 3.4e38 / np.quantile(rec.rho, 0.999)
+        rec.rho = np.ones((n_y, n_z), np.float32)
+        rec(None, 1)
+        rec.accumulate()
+        rec.update(scale)
+        rho = rec.rho
+        infinite = np.isinf(rho)
+        assert 0 < infinite.sum() < 20 and not np.isnan(rho).any()
+        rec(None, 1)
+        img = rec.rho
+    seen = orc.forward_f64(g, *ev, infinite.astype(np.float32), s_z, s_dl) > 0
+    assert 0 < seen.sum() < 3_000
+    kept = [v[~seen] for v in ev]
+    ref = orc.mlem_f64(g, *kept, 1, rho=np.where(infinite, 0.0, rho))
+    assert np.all(img[infinite] == 0.0)
+    assert rel(img, ref) < IMAGE_TOL

@@ -27,8 +27,9 @@ struct hybrid_ctx {
   // returns about ten of them, and with cudaMalloc / cudaFree (which wait for
   // the device and map memory) that was most of its time for short lists
   // (50 000 responses, three iterations and the image: 2.5 ms a pass with
-  // them, 0.53 ms from the pool).  The pool keeps its memory until the
-  // context is destroyed.
+  // them, 0.53 ms from the pool once it has grown, 1.3 ms the first time).  The
+  // pool keeps the most that a list has taken until the context is destroyed or
+  // other memory of it runs short (dalloc).
   cudaMemPool_t pool = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int sm_count = 148;
@@ -107,6 +108,16 @@ template <typename T> cudaError_t ev_alloc(hybrid_ctx* ctx, T** p, size_t bytes)
 template <typename T> void ev_free(hybrid_ctx* ctx, T*& p) {
   EventMemory{ctx->pool, ctx->stream}.free(p);
   p = nullptr;
+}
+
+// Other device memory; the pool's unused part is given back where it is short.
+template <typename T> cudaError_t dalloc(hybrid_ctx* ctx, T** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !ctx->pool) return e;
+  cudaGetLastError();
+  cudaStreamSynchronize(ctx->stream);
+  cudaMemPoolTrimTo(ctx->pool, 0);
+  return cudaMalloc(p, bytes);
 }
 
 inline int64_t lor_index(int64_t first, int64_t second) {
@@ -213,9 +224,12 @@ int order_for_iterations(hybrid_ctx* ctx, int max_planes) {
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
+    ev_free(ctx, ctx->d_frames_iter);
+    // without memory for the order the iterations take the events as they came
+    if (e == cudaErrorMemoryAllocation) return STRIP_OK;
     free_events(ctx);
-    return fail(ctx, e == cudaErrorMemoryAllocation ? STRIP_E_NOMEM : STRIP_E_CUDA,
-                "ordering the frame events: %s", cudaGetErrorString(e));
+    ctx->stats.n_events = ctx->stats.used_pixels = ctx->stats.used_voxels = 0;
+    return fail(ctx, STRIP_E_CUDA, "ordering the frame events: %s", cudaGetErrorString(e));
   }
   return STRIP_OK;
 }
@@ -224,7 +238,7 @@ int order_for_iterations(hybrid_ctx* ctx, int max_planes) {
 // the windowed events, then the others and those the windows left over.
 int enqueue_mlem(hybrid_ctx* ctx, float* acc) {
   const int blocks = ctx->sm_count * mlem_blocks_per_sm();
-  if (!ctx->d_spill) CK(cudaMalloc(&ctx->d_spill, mlem_spill_floats(blocks) * sizeof(float)));
+  if (!ctx->d_spill) CK(dalloc(ctx, &ctx->d_spill, mlem_spill_floats(blocks) * sizeof(float)));
   CK(cudaMemsetAsync(acc, 0, ctx->n_voxels * sizeof(float), ctx->stream));
   const WinSet& ws = ctx->win;
   if (ws.n_events > 0) CK(cudaMemsetAsync(ws.counters, 0, 3 * sizeof(int32_t), ctx->stream));
@@ -234,9 +248,10 @@ int enqueue_mlem(hybrid_ctx* ctx, float* acc) {
                     ctx->stream);
     CK(cudaGetLastError());
   }
+  const Frame* frames = ctx->d_frames_iter ? ctx->d_frames_iter : ctx->d_frames;
   if (ctx->n_events > 0)
-    launch_mlem(ctx->g, geo_view(ctx), ctx->d_sens, ctx->d_frames_iter + ws.n_events,
-                ctx->n_events - ws.n_events, ctx->d_frames_iter, ws.list,
+    launch_mlem(ctx->g, geo_view(ctx), ctx->d_sens, frames + ws.n_events,
+                ctx->n_events - ws.n_events, frames, ws.list,
                 ws.n_events > 0 ? ws.counters + 2 : nullptr, ctx->d_rho_t, acc, ctx->d_spill,
                 blocks, ctx->stream);
   CK(cudaGetLastError());
@@ -276,14 +291,14 @@ int upload_geometry(hybrid_ctx* ctx, int32_t n_detectors, std::vector<float>& se
     len[li] = sg[8];
     used += lend[li] > lbeg[li];
   }
-  CK(cudaMalloc(&ctx->d_md, n_lors * sizeof(float4)));
-  CK(cudaMalloc(&ctx->d_len, n_lors * sizeof(float)));
-  CK(cudaMalloc(&ctx->d_lbeg, n_lors * sizeof(int64_t)));
-  CK(cudaMalloc(&ctx->d_lend, n_lors * sizeof(int64_t)));
-  CK(cudaMalloc(&ctx->d_pix, n_infos * sizeof(short2)));
-  CK(cudaMalloc(&ctx->d_pos, n_infos * sizeof(float)));
-  CK(cudaMalloc(&ctx->d_w_raw, n_infos * sizeof(float)));
-  CK(cudaMalloc(&ctx->d_w, n_infos * sizeof(float)));
+  CK(dalloc(ctx, &ctx->d_md, n_lors * sizeof(float4)));
+  CK(dalloc(ctx, &ctx->d_len, n_lors * sizeof(float)));
+  CK(dalloc(ctx, &ctx->d_lbeg, n_lors * sizeof(int64_t)));
+  CK(dalloc(ctx, &ctx->d_lend, n_lors * sizeof(int64_t)));
+  CK(dalloc(ctx, &ctx->d_pix, n_infos * sizeof(short2)));
+  CK(dalloc(ctx, &ctx->d_pos, n_infos * sizeof(float)));
+  CK(dalloc(ctx, &ctx->d_w_raw, n_infos * sizeof(float)));
+  CK(dalloc(ctx, &ctx->d_w, n_infos * sizeof(float)));
   CK(cudaMemcpyAsync(ctx->d_md, md.data(), n_lors * sizeof(float4), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_len, len.data(), n_lors * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_lbeg, lbeg.data(), n_lors * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));

@@ -358,6 +358,12 @@ cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* fr
     const cudaError_t s = cudaStreamSynchronize(st);
     return r != cudaSuccess ? r : s;
   };
+  // no memory for the windows: the ordered events go without
+  auto no_windows = [&](cudaError_t r) {
+    if (r != cudaErrorMemoryAllocation) return done(r);
+    cudaGetLastError();
+    return done(cudaSuccess);
+  };
 #define STEP(call)                              \
   do {                                          \
     e = (call);                                 \
@@ -396,7 +402,8 @@ cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* fr
   STEP(scan_total(flag, nf, &n_items));
   int32_t* begin = index_out;  // so are the sorted ones (n_items + 1 <= nn)
   k_item_begins<<<grid_for(nf), 256, 0, st>>>(flag, offs, nf, (int32_t)n_items, begin);
-  STEP(mem.alloc(&items_tmp, (size_t)n_items * sizeof(WinItem)));
+  e = mem.alloc(&items_tmp, (size_t)n_items * sizeof(WinItem));
+  if (e != cudaSuccess) return no_windows(e);
   WinItem* items = static_cast<WinItem*>(items_tmp);
   k_item_boxes<<<grid_for(n_items * 32), 256, 0, st>>>(out, begin, (int32_t)n_items, items, flag);
   STEP(scan_total(flag, (int32_t)n_items, &n_tasks));
@@ -408,7 +415,8 @@ cudaError_t order_frames(const GridF& g, const GeometryDev& geo, const Frame* fr
                b_ta = up((size_t)n_tasks * sizeof(WinTask)), b_D = up((size_t)nf * sizeof(double)),
                b_inv = up((size_t)nf * sizeof(float)), b_li = up((size_t)nf * sizeof(int32_t));
   void* own_p = nullptr;
-  STEP(mem.alloc(&own_p, b_ev + b_it + b_ta + b_D + b_inv + b_li + 256));
+  e = mem.alloc(&own_p, b_ev + b_it + b_ta + b_D + b_inv + b_li + 256);
+  if (e != cudaSuccess) return no_windows(e);
   char* own = static_cast<char*>(own_p);
   ws->block = own;
   STEP(cudaMemcpyAsync(own + b_ev, items, (size_t)n_items * sizeof(WinItem),

@@ -410,7 +410,8 @@ __device__ __forceinline__ void pair_item(const LaunchArgs& a, const WorkItem& i
                            PairWalk<CS>(r.run, win.w + ra + 4u * LPE * b,
                                         win.w + rb - 4u * LPE * b), s0, s2);
           auto row = [&](const GaussGradRow& g, float s0, float s2) {
-            if (s0 != 0.0f) {  // rows without pixels have any pref, fz and fdl
+            // rows without pixels have any pref, fz and fdl
+            if (s0 != 0.0f || s2 != 0.0f) {
               grad[0] += w * (double)(g.pref * fmaf(g.fz, s0, 2.0f * a.k.ipsz * s2));
               grad[1] += w * (double)(g.pref * g.fdl * s0);
             }

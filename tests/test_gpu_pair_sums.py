@@ -36,3 +36,19 @@ def test_pixels_that_an_update_made_infinite(accum):
     ref = orc.mlem_f64(g, *kept, 1, rho=np.where(infinite, 0.0, rho))
     assert np.all(img[infinite] == 0.0)
     assert rel(img, ref) < IMAGE_TOL
+
+
+def test_sigma_gradient_of_rows_whose_values_cancel():
+    """A signed image whose sum over every full row is exactly zero: the rows
+    still have a derivative.  The sigma_z makes neighbouring kernel values
+    powers of two apart, so the binary32 sums cancel without a rounding."""
+    s_z, s_dl = 1.6986435651779175, 10.0
+    g = orc.geometry(100.0, 200.0, 64, 64, 1.0, 1.0, s_z, s_dl)
+    ev = [np.zeros(1, np.float32)] * 3
+    rho = np.zeros((64, 64), np.float32)
+    rho[:, [30, 33]], rho[:, [31, 32]] = 2.0, -1.0
+    with sm.Reconstruction(sm.Scanner(100.0, 200.0, 64, 64, 1.0, 1.0, s_z, s_dl)) as rec:
+        rec.set_events(*ev)
+        got = rec.grad_sigma(rho, np.ones(1), s_z, s_dl)
+    want = orc.grad_sigma_f64(g, *ev, rho, np.ones(1), s_z, s_dl)
+    assert abs(got[0] / want[0] - 1) < IMAGE_TOL

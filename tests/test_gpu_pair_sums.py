@@ -52,3 +52,27 @@ def test_sigma_gradient_of_rows_whose_values_cancel():
         got = rec.grad_sigma(rho, np.ones(1), s_z, s_dl)
     want = orc.grad_sigma_f64(g, *ev, rho, np.ones(1), s_z, s_dl)
     assert abs(got[0] / want[0] - 1) < IMAGE_TOL
+
+
+def test_binary64_sums_take_the_rows_one_by_one():
+    """Three pixels of one column, the first two in rows of one pair: the third
+    cancels the first and leaves the second, which a binary32 sum of the first
+    two would have rounded."""
+    n, s_z, s_dl = 64, 5.0, 10.0
+    ev = [np.zeros(1, np.float32)] * 3
+    with sm.Reconstruction(sm.Scanner(100.0, 200.0, n, n, 1.0, 1.0, s_z, s_dl),
+                           accumulation=sm.ACCUM_FP64) as rec:
+        rec.set_events(*ev)
+
+        def forward(values):  # rows 32 and 31: the event's middle pair
+            rho = np.zeros((n, n), np.float32)
+            for row, v in values:
+                rho[row, 30] = v
+            return rec.forward(rho, s_z, s_dl)[0]
+
+        k = {row: forward([(row, 1.0)]) for row in (32, 31, 33)}
+        small = np.float32(1.1e-6)
+        third = np.float32(-k[32] / k[33])
+        rows = [(32, np.float32(1.0)), (31, small), (33, third)]
+        want = sum(float(np.float32(k[r]) * v) for r, v in rows)
+        assert abs(forward(rows) - want) < 1e-12 * k[32]

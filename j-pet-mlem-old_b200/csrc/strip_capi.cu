@@ -232,8 +232,10 @@ Tiling choose_tiling(const strip_ctx* ctx, int max_w, int max_h) {
     // Tall boxes: the tile's rows cut to what the tall stride leaves beside
     // the halos (28 or more at 128 rows).  The row-major form stays possible
     // for the kernels that take it.  Around smaller boxes such windows come
-    // of large tiles; those stay row-major.  (126-row boxes, 4e5 events, 300 x
-    // 437 pixels of 1 mm: five iterations 25.6 ms row-major, 14.2 ms here.)
+    // of large tiles; those stay row-major.  (126-row boxes, 2e6 events, 300 x
+    // 437 pixels of 1 mm: three iterations 25.6 ms row-major, 14.2 ms here.  The
+    // AnalyticKernel, row-major either way, loses nothing by the cut: 5e5 events
+    // 10.4 ms a pass with 32 rows a tile, 10.2 with 30.)
     t.cs = kTallStride;
     t.TY = std::min(t.TY, kTallStride - 2 * t.HY);
     t.WYmax = std::min(n_y, t.TY + 2 * t.HY);
@@ -275,11 +277,8 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
   unsigned long long* d_hist = nullptr;
   float *ozu = nullptr, *ozd = nullptr, *odl = nullptr;
   int64_t* operm = nullptr;
-  // The old events' packs make room: a binning needs 72 bytes an event at its
-  // peak (96 in a batch, whose graph reads them until it is destroyed).
   const bool had_packs = ctx->d_packs != nullptr;
   EventPack* packs = nullptr;
-  if (ctx->in_batch.use_count() == 1) ev_free(ctx, ctx->d_packs);
   auto cleanup = [&]() {
     ev_free(ctx, packs);
     ev_free(ctx, boxes);
@@ -450,12 +449,17 @@ int bin_events(strip_ctx* ctx, const float* zu, const float* zd,
     if (e == cudaSuccess) e = ev_alloc(ctx, &qzd, nb * sizeof(float));
     if (e == cudaSuccess) e = ev_alloc(ctx, &qdl, nb * sizeof(float));
     if (e == cudaSuccess) e = ev_alloc(ctx, &qperm, nb * sizeof(int64_t));
-    // a context that has used packs gets the new ones on the way, given memory (a
-    // launch of their own: 661 against 653 us from 2e4 events to the image)
-    if (e == cudaSuccess && had_packs &&
-        ev_alloc(ctx, &packs, nb * sizeof(EventPack)) != cudaSuccess) {
-      cudaGetLastError();
-      packs = nullptr;
+    // A context that has used packs gets the new ones on the way, given memory (a
+    // launch of their own: 661 against 653 us from 2e4 events to the image), in
+    // the old ones' place: 96 bytes an event at the binning's peak.  (Freed before
+    // the binning, the pool cuts their block up and grows again and again: 2e7
+    // events 9.3 to 46 ms instead of 7.5.)
+    if (e == cudaSuccess && had_packs) {
+      release_packs(ctx);
+      if (ev_alloc(ctx, &packs, nb * sizeof(EventPack)) != cudaSuccess) {
+        cudaGetLastError();
+        packs = nullptr;
+      }
     }
     if (e == cudaSuccess)
       e = launch_item_order(ctx->s, t, d_items, (int)items.size(), ozu, ozd, odl, operm, qzu,
@@ -1289,11 +1293,25 @@ int ctx_fail(strip_ctx* ctx, int code, const char* msg) {
   return fail(ctx, code, "%s", msg);
 }
 
+// Frees the packs (a launch that needs them makes them again), unless a batch's
+// graph reads them.
+bool release_packs(strip_ctx* ctx) {
+  if (!ctx->d_packs || ctx->in_batch.use_count() > 1) return false;
+  ev_free(ctx, ctx->d_packs);
+  return true;
+}
+
+// The packs make room where memory is short, so that they cost no event list its
+// place.
 cudaError_t ev_alloc_bytes(strip_ctx* ctx, void** p, size_t bytes) {
-  *p = nullptr;
-  if (ctx->pool) return cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), ctx->pool,
-                                                ctx->stream);
-  return cudaMalloc(p, std::max<size_t>(bytes, 16));
+  for (;;) {
+    *p = nullptr;
+    const size_t n = std::max<size_t>(bytes, 16);
+    const cudaError_t e = ctx->pool ? cudaMallocFromPoolAsync(p, n, ctx->pool, ctx->stream)
+                                    : cudaMalloc(p, n);
+    if (e != cudaErrorMemoryAllocation || !release_packs(ctx)) return e;
+    cudaGetLastError();
+  }
 }
 
 void ev_free_ptr(strip_ctx* ctx, void* p) {

@@ -76,6 +76,7 @@ int ctx_fail(strip_ctx* ctx, int code, const char* msg);
 // context's stream; plain cudaMalloc / cudaFree without a pool).
 cudaError_t ev_alloc_bytes(strip_ctx* ctx, void** p, size_t bytes);
 void ev_free_ptr(strip_ctx* ctx, void* p);
+bool release_packs(strip_ctx* ctx);
 template <class T>
 cudaError_t ev_alloc(strip_ctx* ctx, T** p, size_t bytes) {
   return ev_alloc_bytes(ctx, reinterpret_cast<void**>(p), bytes);

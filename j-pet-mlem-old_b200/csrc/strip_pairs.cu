@@ -8,10 +8,10 @@
 // runs are equally long to within a pixel or two, and everything about them is
 // one f32x2 operation: the exact set arithmetic, the closed-form run ends,
 // the kernel constants, and the walks E <- E R, R <- R q (a step is one pixel
-// of each row).  Bound by instruction issue (80 % issue-active, the FMA pipe at
-// 51 %).  With one row per lane the set-up of the rows was a third of the MLEM
-// kernel; warp instructions an event at the 800 x 400 benchmark 928 -> 775,
-// 4e6 events 4.39 -> 3.47 ms a pass (forward 2.31 -> 1.93, adjoint 2.65 ->
+// of each row).  Bound by instruction issue (79 % issue-active, the FMA pipe at
+// 51 %, the shared-memory pipe at 61 %).  With one row per lane the set-up of the
+// rows was a third of the MLEM kernel; warp instructions an event at the 800 x
+// 400 benchmark 928 -> 767, 4e6 events 4.39 -> 3.47 ms a pass (forward 2.31 -> 1.93, adjoint 2.65 ->
 // 2.22).  Sixteen lanes an event issue more (943; they serve boxes above 80
 // rows), and 384 threads of 80 registers without spills run slower (4.1 ms).
 //
@@ -519,19 +519,23 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
     for (int q = threadIdx.x; q < kMaxItemEvents / 32; q += blockDim.x) s_fb_bits[q] = 0u;
   const int lane = threadIdx.x & 31;
   float wsum = 0.0f;
-  bool odd = false;  // a pixel below zero, infinite or NaN
+  float wmin = 0.0f;  // the least pixel below zero
   each_pixel<true>(wxn, wyn, lane, [&](int r, int c) {
     if (kReads) {
       const float v = a.rho[(int64_t)(wy0 + r) * a.s.n_z + wx0 + c];
       s_w[c * CS + r] = v;
       if (OP == OP_MLEM) {
         wsum += v;
-        odd |= !(v >= 0.0f && v <= 3.402823466e38f);
+        wmin = fminf(wmin, v);
       }
     }
     if (kWrites) s_acc[c * CS + r] = 0.0f;
   });
-  odd = __syncthreads_or(odd);
+  bool negative = false;
+  if constexpr (OP == OP_MLEM)
+    negative = __syncthreads_or(wmin < 0.0f);
+  else
+    __syncthreads();
   PairWin win{(uint32_t)__cvta_generic_to_shared(s_w), (uint32_t)__cvta_generic_to_shared(s_acc),
               wx0, wy0, 1.0f};
   // groups of events per counter step: fewer for small items, so that every
@@ -573,7 +577,6 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
   } else if constexpr (OP == OP_ADJOINT) {
     // addends below 2^22 (adjoint_shift); without negative weights the
     // subnormal conversion gives the same integers without the subtractions
-    bool negative;
     const int fshift = adjoint_shift(a, it, lane, &negative);
     win.unit = exp2f((float)fshift);
     if (negative)
@@ -634,9 +637,9 @@ __device__ __forceinline__ void pair_tile_item(const LaunchArgs& a, const WorkIt
     if (n_weighted > 0) {
       const int fs = fixed_shift(n_weighted);
       win.unit = exp2f((float)fs);
-      // K rho / D <= 1: addends up to the unit; over images that updates made
-      // infinite, say, they may be anything, which cvt.rni clamps
-      if (fs <= 23 && !odd)
+      // K rho / D <= 1: addends up to the unit; over pixels below zero, infinite
+      // (updates can make some) or NaN they may be anything, which cvt.rni clamps
+      if (fs <= 23 && !negative && wmean <= 3.402823466e38f)
         pair_item<OP, ACC, LPE, NB, CS, true, kAddWeightedSubnormal>(a, it, win, lane, grab,
                                                                  s_next_group, only);
       else
@@ -660,7 +663,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == kPairWide ? 1 : 2)
 // Blocks of row pairs held through both passes: 5 blocks of 8 pairs (80 rows)
 // or 4 of 16 (128 rows).  Boxes of at most 80 rows take 8 lanes an event; the
 // windows of taller ones have the tall column stride where they need it
-// (tile_column_stride).
+// (choose_tiling).
 constexpr int kBlocks8 = 5, kBlocks16 = 4;
 static_assert(16 * kBlocks8 == kPairRows8 && 32 * kBlocks16 == kPairRows16, "row-pair layouts");
 

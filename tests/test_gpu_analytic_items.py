@@ -34,3 +34,27 @@ def test_small_items(case, n, item):
         assert rec.stats()["n_overflow"] == 0
     assert rel(img, orc.mlem_f64(g, *ev, 2, mode=1)) < TOL
     assert rel(y, orc.forward_f64(g, *ev, rho, s_z, s_dl, mode=1)) < TOL
+
+
+def test_batch_of_tall_and_short_boxes():
+    """Boxes of 81 to 128 rows have tilings of the row-pair kernels' tall columns,
+    which the AnalyticKernel reads row-major: beside column-major and row-major
+    members, in one batch."""
+    recs, refs = [], []
+    try:
+        for case in (CASES[4], CASES[0], CASES[5], (150.0, 300.0, 190, 211, 1.0, 6.0, 44.0)):
+            R, L, n_y, n_z, p, s_z, s_dl = case
+            ev = events(case, 1_201, 13)
+            rec = sm.Reconstruction(sm.Scanner(R, L, n_y, n_z, p, p, s_z, s_dl),
+                                    mode=sm.MODE_GPU)
+            recs.append(rec)
+            rec.set_events(*ev)
+            g = orc.geometry(R, L, n_y, n_z, p, p, s_z, s_dl)
+            refs.append(orc.mlem_f64(g, *ev, 2, mode=1))
+        with sm.Batch(recs, mode=sm.MODE_GPU) as batch:
+            batch(2)
+        for rec, ref in zip(recs, refs):
+            assert rel(rec.rho, ref) < TOL
+    finally:
+        for rec in recs:
+            rec.close()

@@ -690,7 +690,7 @@ def ours(args, rank, world, local_rank):
             "hbm": {"achieved_gbs": hbm_achieved, "peak_gbs": hbm_peak,
                     "frac": hbm_achieved / hbm_peak if hbm_peak else None,
                     "peak_source": "MEASURED_PEAKS.json hbm_gbs"},
-            "kernel": "k_tile (tile-window MLEM kernel)",
+            "kernel": "k_pair_tile (tile-window MLEM kernel, row pairs)",
             "work_model": "10 flops per bbox pixel + 18 per in-ellipse pixel",
             "bbox_pixels_per_iter": work_bb.value, "ellipse_pixels_per_iter": work_in.value,
             "tile_ms_per_step": tile_ms / args.steps,

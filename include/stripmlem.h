@@ -276,8 +276,9 @@ int strip_set_schedule(strip_ctx* ctx, int tile, int grab);
 /* Largest tile work item, in events (1..8000); 0 (the default) picks it per
  * binning: enough items for about eight waves of the device, at least 2048
  * and at most 8000 events, the last wave's worth of each subset's items cut
- * into quarter pieces; subsets of up to 1.2e6 events in items of 128 to 1024
- * events, uncut.  Re-bins the events when the context has some.
+ * into quarter pieces; with column-major windows and outside batches, subsets
+ * of up to 1.2e6 events in items of 128 to 1024 events, uncut.  Re-bins the
+ * events when the context has some.
  * The item size changes the work decomposition and the fixed-point scale of
  * each item's window, not the result beyond rounding; a small event set
  * binned with 8000-event items runs the arithmetic of a large one. */

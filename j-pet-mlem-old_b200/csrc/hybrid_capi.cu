@@ -191,15 +191,12 @@ void free_events(hybrid_ctx* ctx) {
 // per iteration of k_mlem -> windowed): 60, 2e5: 0.74, 0.281 -> 0.286;
 // 100, 2e5: 0.73, 0.733 -> 0.645; 160, 2e5: 0.78, 2.22 -> 1.95; 80, 1e5: 1.4,
 // 0.246 -> 0.353; 100, 5e4: 1.7, 0.197 -> 0.357; 100, 2e6: 0.12, 6.97 -> 2.45;
-// so below HYBRID_WIN_RATIO entries a voxel.  Lists of fewer than
-// HYBRID_WIN_EVENTS_PER_LOR events per LOR with pixel infos lie beyond that
+// so below kWinRatio entries a voxel.  Lists of fewer than
+// kWinEventsPerLor events per LOR with pixel infos lie beyond that
 // (5e4 to 1e5 responses there) and are not binned at all.
-#ifndef HYBRID_WIN_EVENTS_PER_LOR
-#define HYBRID_WIN_EVENTS_PER_LOR 8
-#endif
-#ifndef HYBRID_WIN_RATIO
-#define HYBRID_WIN_RATIO 0.74
-#endif
+constexpr int kWinEventsPerLor = 8;
+constexpr double kWinRatio = 0.74;
+
 // Orders the frame events for the iterations: LOR by LOR, and within a LOR by
 // plane slab when the windows pay.  The order of the additions into the
 // volume changes only the binary32 rounding of the sums.
@@ -213,12 +210,12 @@ int order_for_iterations(hybrid_ctx* ctx, int max_planes) {
   cudaError_t e = ev_alloc(ctx, &ctx->d_frames_iter, ctx->n_events * sizeof(Frame));
   if (e == cudaSuccess)
     e = order_frames(ctx->g, geo_view(ctx), ctx->d_frames, (int32_t)ctx->n_events,
-                     ctx->n_events >= HYBRID_WIN_EVENTS_PER_LOR * ctx->n_lors_used
+                     ctx->n_events >= kWinEventsPerLor * ctx->n_lors_used
                          ? plan_windows(ctx->g, max_planes) : WinPlan{},
                      ctx->d_frames_iter, &ctx->win,
                      EventMemory{ctx->pool, ctx->stream});
   if (e == cudaSuccess &&
-      (double)ctx->win.entries >= HYBRID_WIN_RATIO * (double)ctx->stats.used_voxels) {
+      (double)ctx->win.entries >= kWinRatio * (double)ctx->stats.used_voxels) {
     ev_free(ctx, ctx->win.block);
     ctx->win = WinSet{};
   }

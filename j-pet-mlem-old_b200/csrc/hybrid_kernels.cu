@@ -171,8 +171,8 @@ __device__ __forceinline__ float voxel_kw(const GridF& g, const Frame& f, const 
   return t4.x * exp2f(-0.7213475204444817f * bcb) * is;  // exp(-bcb / 2)
 }
 
-// Events frames[0 .. n_frames) and then the *n_list events that k_mlem_win
-// left to this kernel (list; both null without windows).
+// Events frames[0 .. n_frames) and then the *n_list events that the windowed
+// kernels left to this one (list; both null without windows).
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 k_mlem(const GridF g, const GeometryDev geo, const float* __restrict__ sens,
        const Frame* __restrict__ frames, int64_t n_frames, const Frame* __restrict__ win_frames,
@@ -310,14 +310,8 @@ k_mlem(const GridF g, const GeometryDev geo, const float* __restrict__ sens,
 // were.
 constexpr int kWinStride = 66;  // words between planes: 64 infos + 2 (lane =
                                 // plane stores of row pairs hit all banks)
-#ifndef HYBRID_WIN_WARPS
-#define HYBRID_WIN_WARPS 4
-#endif
-#ifndef HYBRID_WIN_CTAS
-#define HYBRID_WIN_CTAS 4
-#endif
-constexpr int kWinWarps = HYBRID_WIN_WARPS;  // per CTA (they share nothing)
-constexpr int kWinCtas = HYBRID_WIN_CTAS;    // per SM
+constexpr int kWinWarps = 4;  // per CTA (they share nothing)
+constexpr int kWinCtas = 4;   // per SM
 constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ float ex2(float x) {
@@ -344,7 +338,7 @@ __device__ __forceinline__ WinConst win_const(const GridF& g) {
   return k;
 }
 
-// The frame events' window form (win_pack in hybrid_internal.h).
+// The frame events' window form (WinEvent in hybrid_internal.h).
 __global__ void k_win_events(const GridF g, const GeometryDev geo,
                              const Frame* __restrict__ frames, int32_t n, WinEvent* out) {
   for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -409,7 +403,7 @@ __device__ __forceinline__ float rcp(float x) {
 }
 
 // inv_sens of two pixels at the plane with half_L - z = lm and half_L + z =
-// lp, times m: atan2_pos's polynomial in packed arithmetic.
+// lp, times m: atan2_pos in packed arithmetic (the same coefficients).
 __device__ __forceinline__ float2 inv_sens2(float lm, float lp, float2 ra, float2 rb, float2 m) {
   constexpr float kAtan[8] = {-0.0040545654483139515f, 0.021862952038645744f, -0.0559123195707798f, 0.0964219719171524f,
                               -0.1390862911939621f, 0.19946566224098206f, -0.33329859375953674f, 0.9999993443489075f};

@@ -35,7 +35,7 @@ constexpr int kNarrowSmem = kNarrowSmemBytes;
 constexpr int kClasses = 8;
 inline int class_windows(int c) { return c >> 1; }
 // Members with at least this many work items per SM get a tile launch of
-// their own (k_tile, arguments in constant parameter space) instead of
+// their own (arguments in constant parameter space) instead of
 // joining the persistent launch, whose per-member arguments are indexed at
 // run time and cost registers; the own launches run on kSideStreams streams
 // forked from the batch stream, beside the persistent launches that fill

@@ -1199,18 +1199,18 @@ __global__ void k_bin_scatter(const int* keys, int64_t n, const float* zu,
 }
 
 // Orders the events of each work item for the column-major windows' banks.
-// A lane's bank there is its row's, (row - wy0) mod 32, and the rows of a
-// row block, ranked middle-out from the event's middle row m, cover a fixed
-// set of residues around m: for 16-row blocks half of Z_32 whose other half
-// is the same set around m + 16, for 8-row blocks a quarter whose shifts by
-// 8, 16 and 24 tile Z_32.  So the item is laid out in quads of events whose
-// middle rows are v, v + 16, v + 8 and v + 24 mod 32 (the half-warp pairs of
-// MLEM take (v, v + 16) and (v + 8, v + 24), the quarter-warps of the
-// forward and adjoint all four), then pairs (v, v + 16) of the events left,
-// then the rest.  Within a middle-row class the events go by size (box rows,
-// eight steps of a sixteenth of the tallest), so that the events of a quad are
-// alike and their walks equally long.  One CTA per item; the order within a
-// class and size is that of the atomics.  The results change only by the order of the binary32
+// A lane's bank there is its row's, (row - wy0) mod 32.  The row-pair kernels'
+// eight lanes of an event read eight neighbouring rows an instruction, above or
+// below its middle row m (sixteen lanes: sixteen rows), a quarter of Z_32 whose
+// shifts by 8, 16 and 24 are the rest (a half).  So the item is laid out in
+// quads of events whose middle rows are v, v + 16, v + 8 and v + 24 mod 32, which
+// share a warp (with sixteen lanes the pairs (v, v + 16) and (v + 8, v + 24)),
+// then pairs (v, v + 16) of the events left, then the rest.  k_tile's half-warps
+// and quarter-warps, whose blocks are ranked middle-out, gain the same way.
+// Within a middle-row class the events go by size (box rows, eight steps of a
+// sixteenth of the tallest), so that the events of a quad are alike and their
+// walks equally long.  One CTA per item; the order within a class and size is
+// that of the atomics.  The results change only by the order of the binary32
 // sums.
 __global__ void k_item_order(ScannerF s, Tiling t, const WorkItem* __restrict__ items,
                              const float* __restrict__ zu, const float* __restrict__ zd,
